@@ -5,8 +5,8 @@ Knobs, each chosen by timing on the device (CUDA events on the launching stream)
 * ``team`` — lanes per quartet of the register kernel (light classes): each quartet's
   primitive loop is split over `team` lanes (1..32) and the partial [e0|f0] summed with warp
   shuffles.  Few primitives favour small teams, heavily contracted quartets large ones.
-* ``variant`` — heavy classes that have both kernels: the split register kernel (0) or the
-  line-factorised kernel (1).
+* ``variant`` — the heavy classes' kernel: the quadrature kernel (0); the others (1, 2) are
+  slower on every workload's blocks together and round differently, so the tuner offers 0 only.
 * ``ctas_per_sm`` — the register kernel's grid cap, in resident CTAs per SM (2..16): more
   CTAs shorten the tail of a block, fewer stage the Boys table fewer times.
 * ``streams`` — how many concurrent streams the class blocks of a call are spread over
@@ -35,6 +35,7 @@ __all__ = ["autotune", "apply_cache", "cache_path", "TEAMS", "CTAS", "STREAMS"]
 TEAMS = (1, 2, 4, 8, 16, 32)
 CTAS = (2, 4, 8, 16)
 STREAMS = (1, 2, 4, 6, 8, 12, 16)
+VARIANTS = (0,)
 
 
 def light_class(cls4):
@@ -154,9 +155,9 @@ def autotune(shells, coord_types=None, reps=3, teams=TEAMS, ctas=CTAS, streams=S
     def set_cap(k, c):
         cap[k] = c
         db.set_block_config(k, var[k], c)
-    t_var = _sweep(db, blocks, heavy, (0, 1), set_var, reps)
+    t_var = _sweep(db, blocks, heavy, VARIANTS, set_var, reps)
     for k in heavy:
-        set_var(k, int(np.argmin(t_var[:, k])))
+        set_var(k, VARIANTS[int(np.argmin(t_var[:, k]))])
         chosen["v:" + keys[k]] = var[k]
     timings["variant"] = t_var
     t_cap = _sweep(db, blocks, light, ctas, set_cap, reps)

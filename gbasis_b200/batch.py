@@ -102,7 +102,7 @@ class EriBatch:
         of the heavy types, then the grid cap of the register-kernel types; keep the fastest
         and store the choices in the tuning cache."""
         import json
-        from .autotune import CTAS, TEAMS, _key, _load, cache_path, light_class
+        from .autotune import CTAS, TEAMS, VARIANTS, _key, _load, cache_path, light_class
         teams = TEAMS if teams is None else teams
         L = _engine.lib()
         types = self.types()
@@ -139,9 +139,9 @@ class EriBatch:
                 best = teams[int(np.argmin(times[:, k]))]
                 self.set_team(k, best)
                 chosen[keys[k]] = best
-            t_var = sweep(heavy, (0, 1), set_var)
+            t_var = sweep(heavy, VARIANTS, set_var)
             for k in heavy:
-                set_var(k, int(np.argmin(t_var[:, k])))
+                set_var(k, VARIANTS[int(np.argmin(t_var[:, k]))])
                 chosen["v:" + keys[k]] = var[k]
             t_cap = sweep(light, CTAS, set_cap)
             for k in light:

@@ -13,7 +13,6 @@ integrals (spherical), ``batch512`` every molecule's full tensor (one graph of b
 from __future__ import annotations
 
 import ctypes
-import os
 import sys
 
 import numpy as np
@@ -26,16 +25,9 @@ __all__ = ["block_rows", "kernel_of", "markdown"]
 
 
 def kernel_of(cls4):
-    """Which kernel runs a class's store mode: ``register`` (light classes), ``split``
-    (heavy classes whose row ranges fit threads) or ``line``."""
+    """Which kernel runs a class by default: ``register`` (light classes) or ``quadrature``."""
     from .autotune import light_class
-    if light_class(cls4):
-        return "register"
-    here = os.path.join(os.path.dirname(os.path.abspath(__file__)), "csrc")
-    if here not in sys.path:
-        sys.path.insert(0, here)
-    import gen_lines  # the generator that chose the kernels at build time
-    return "split" if gen_lines.split_ok(tuple(cls4)) else "line"
+    return "register" if light_class(cls4) else "quadrature"
 
 
 def _row(cls4, team, avg, nq, ms, peak):

@@ -56,9 +56,13 @@ LINES_DEPS = ("gbx_common.cuh", "errors.h", "coop.cuh", "coop_tail.cuh", "lines_
               "eri_kernels.cuh", "_gen/eri_gen.cuh")
 
 
+RYS_DEPS = ("gbx_common.cuh", "errors.h", "rys_kernel.cuh", "eri_kernels.cuh", "_gen/eri_gen.cuh")
+
+
 def _deps_mtime(src):
     base = os.path.basename(src)
     deps = (KERNEL_DEPS if base.startswith("eri_cls") else
+            RYS_DEPS if base.startswith("rys_") else
             LINES_DEPS if base.startswith("lines_") else
             KERNEL_DEPS + HOST_DEPS if base in ("one_elec.cu", "boys_eval.cu") else HOST_DEPS)
     m = os.path.getmtime(os.path.join(ROOT, "include", "gbx_eri.h"))

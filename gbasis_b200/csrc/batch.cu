@@ -34,7 +34,7 @@ struct BatchType {
   long long n = 0, work_off = 0;
   double avg_prims = 1.0;
   int team = 1;
-  int variant = 0;      // heavy classes with both kernels: 0 split, 1 line kernel
+  int variant = 0;      // heavy classes' kernel (EriLaunch::variant)
   int ctas_per_sm = 8;  // grid cap of the register kernel (resident-CTA multiples of the SMs)
   long long* d_base = nullptr;   // per molecule: block base in the batch compact store
   long long* d_ncols = nullptr;  // per molecule: pair functions of the ket class

@@ -134,7 +134,8 @@ struct EriLaunch {
   // two-electron operator: 0 = 1/r, 1 = erf(omega r)/r, 2 = erfc(omega r)/r
   int potential;
   double omega;
-  // heavy classes that have both kernels: 0 = split register kernel, 1 = line kernel
+  // heavy classes: 0 = quadrature kernel, 1 = line kernel, 2 = split register kernel (classes that
+  // have one) or the line kernel's group form
   int variant;
   // work counter of this launch, zero before it starts: in the heavy-class kernels warps (split
   // kernel: CTAs) take their next quartets from it with atomicAdd, so that a CTA that becomes

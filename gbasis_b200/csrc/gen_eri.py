@@ -446,6 +446,9 @@ def emit_sources(outdir, lmax):
     import gen_lines
     lfiles, launchers = gen_lines.emit_sources(outdir, heavy)
     files += lfiles
+    import gen_rys
+    rfiles, rlaunchers = gen_rys.emit_sources(outdir, heavy)
+    files += rfiles
     lines = ["// Generated by gen_eri.py: (la,lb,lc,ld) -> class kernel launcher.",
              "#include <cstdlib>",
              "#include <cstring>",
@@ -459,7 +462,15 @@ def emit_sources(outdir, lmax):
                      "int, cudaStream_t);")
     for c in heavy:
         lines.append(f"int {launchers[c]}(const EriLaunch& a, cudaStream_t st);")
-    lines.append("// Heavy classes run the line-factorised kernel; GBX_HEAVY_KERNEL=interp selects the")
+        lines.append(f"int {rlaunchers[c]}(const EriLaunch& a, cudaStream_t st);")
+    lines.append("// Heavy classes run the quadrature kernel (eri_rys).  The block's variant knob selects the")
+    lines.append("// line kernel (1) or (2) its group form or, for the classes that have one, the split kernel:")
+    lines.append("// a thread per quartet, which is faster on long lists of quartets with equal primitive")
+    lines.append("// counts (33,000 to 120,000 quartets of 45 to 60 primitive quartets: 1.4 to 1.8 times,")
+    lines.append("// (pf|sp) 0.70 against 1.28 ms) and slower on short or uneven ones (7,000 to 20,000: 1.2")
+    lines.append("// to 1.9 times, (pd|sd) 0.31 against 0.19 ms).  The rule does not look at the list: a")
+    lines.append("// quartet's value must not depend on the list it is in.")
+    lines.append("// GBX_HEAVY_KERNEL=interp selects the")
     lines.append("// program-interpreting cooperative kernel instead (read once per process).")
     lines.append("static bool heavy_interp() {")
     lines.append('  static const bool v = [] { const char* e = std::getenv("GBX_HEAVY_KERNEL");')
@@ -476,7 +487,7 @@ def emit_sources(outdir, lmax):
     for j, c in enumerate(heavy):
         key = ((c[0] * 8 + c[1]) * 8 + c[2]) * 8 + c[3]
         lines.append(f"    case {key}: return heavy_interp() ? launch_coop({j}, a, st) : "
-                     f"{launchers[c]}(a, st);")
+                     f"a.variant == 0 ? {rlaunchers[c]}(a, st) : {launchers[c]}(a, st);")
     lines.append("    default: break;")
     lines.append("  }")
     lines.append('  return set_error(GBX_ERR_UNSUPPORTED, "no kernel for class (%d %d|%d %d)", '

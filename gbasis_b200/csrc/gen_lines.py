@@ -389,7 +389,7 @@ def emit_sources(outdir, heavy, nfiles=12):
             launchers[c] = name
             out.append(f"int {name}(const EriLaunch& a, cudaStream_t st) {{")
             if split_ok(c):
-                out.append(f"  if (a.variant == 0) return launch_split_t<SplitCls_{tag}>(a, st);")
+                out.append(f"  if (a.variant == 2) return launch_split_t<SplitCls_{tag}>(a, st);")
             out.append(f"  return launch_lines_t<LinesCls_{tag}>(a, kCoopMeta[{j}], st);")
             out.append("}")
         out.append("}  // namespace gbx")
@@ -464,13 +464,12 @@ def emit_tail(cls):
 
 # ------------------------------------------------------------------- split register kernel
 GROUP_W = 4         # warps of the group form's CTA (one quartet per CTA)
-SPLITS = (4, 8)     # warps of a CTA, each computing one part of the targets
+SPLIT_S = 4         # warps of a CTA, each computing one part of the targets
 SPLIT_MAX_ACC = 64  # accumulators per thread in a part
-SPLIT_MAX_OPS = 500  # recursion operations per part with 4 parts
-# with 8 parts: every class of 620 < ops <= 750 (and every one of 500 < ops <= 620 with more
-# than 40 accumulators) was checked spill-free with ptxas on sm_100a (226-252 registers);
-# 906 ops spilled 220-530 bytes
-SPLIT_MAX_OPS_8 = 750
+# recursion operations per part: what compiles without spills (ptxas, sm_100a).  Larger classes
+# (parts of 500 to 750 operations, 8 warps) ran 1.7 to 2.1 times slower here than on the
+# quadrature kernel: 8 warps of different straight-line code, 12 KB each, miss the instruction cache
+SPLIT_MAX_OPS = 500
 SPLIT_MAX_L = 7
 
 
@@ -483,10 +482,9 @@ def split_parts(cls, S):
 
 
 def split_ok(cls):
-    """Number of parts (warps) of the split kernel for the class, or 0: the smallest S whose
-    parts fit a thread's registers (at most SPLIT_MAX_ACC accumulators and SPLIT_MAX_OPS
-    recursion operations per part, or 620 operations with at most 40 accumulators, or with 8
-    parts SPLIT_MAX_OPS_8; beyond that the parts spill, as measured with ptxas on sm_100a)."""
+    """Number of parts (warps) of the split kernel for the class, or 0: the parts have to fit a
+    thread's registers (at most SPLIT_MAX_ACC accumulators and SPLIT_MAX_OPS recursion operations
+    per part, or 620 operations with at most 40 accumulators)."""
     return _split_ok(tuple(cls))
 
 
@@ -498,17 +496,14 @@ def _split_ok(cls):
     F = G.comps_range(lc, lc + ld)
     if not (sum(cls) <= SPLIT_MAX_L and tail_fits(cls)):
         return 0
-    for S in SPLITS:
-        parts = split_parts(cls, S)
-        if not all(e1 > e0 for e0, e1 in parts):
-            continue
-        acc = max(e1 - e0 for e0, e1 in parts) * len(F)
-        if acc > SPLIT_MAX_ACC:
-            continue
-        ops = max(_part_gen(cls, E[e0:e1], F).op_count() for e0, e1 in parts)
-        if ops <= SPLIT_MAX_OPS or (acc <= 40 and ops <= 620) or (S == 8 and ops <= SPLIT_MAX_OPS_8):
-            return S
-    return 0
+    parts = split_parts(cls, SPLIT_S)
+    if not all(e1 > e0 for e0, e1 in parts):
+        return 0
+    acc = max(e1 - e0 for e0, e1 in parts) * len(F)
+    if acc > SPLIT_MAX_ACC:
+        return 0
+    ops = max(_part_gen(cls, E[e0:e1], F).op_count() for e0, e1 in parts)
+    return SPLIT_S if ops <= SPLIT_MAX_OPS or (acc <= 40 and ops <= 620) else 0
 
 
 def _part_gen(cls, E, F):

@@ -533,20 +533,14 @@ int launch_lines_t(const EriLaunch& a, const CoopMeta& m, cudaStream_t st) {
   }
   if (s) return s;
   if constexpr (C::kGroup) {
-    // group form (a.variant 2), or by default (a.variant 0) for classes whose ket pair has no
-    // s shell first (LC >= 1); not for the Schwarz diagonal (mode 1).  Measured per class on the
-    // 20-atom chain's unique integrals, blocks one after another: the group form took up to
-    // 55 % off the classes with LC >= 1 ((ff|df) 107 -> 56 ms, (ff|ff) 54 -> 25, (ff|pf)
-    // 84 -> 65; three within 5 % either way) and cost up to 100 % on most LC = 0 classes
-    // ((df|sp) 77 -> 156 ms)
+    // group form (a.variant 2); not for the Schwarz diagonal (mode 1)
     CoopArgs G;
     G.a = a;
     G.m = m;
     size_t gsmem = 0;
     int one = 1;
     // the kernel's own 8-byte ticket slot sits in static shared memory beside the plan's
-    const bool group = a.mode != 1 &&
-                       (a.variant == 2 || (a.variant == 0 && C::LC >= 1)) &&
+    const bool group = a.mode != 1 && a.variant == 2 &&
                        coop_plan(m, (long long)C::kW + C::kY + C::L + 1, G, gsmem, one,
                                  16 / kLinesGroupW, true, 1) == GBX_OK &&
                        (long long)gsmem + 64 <= kCoopMaxSmem;

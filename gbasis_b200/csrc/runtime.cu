@@ -73,6 +73,10 @@ void boys_host_table(double* h) {
 int boys_table(int device, const double** out) {
   std::lock_guard<std::mutex> lk(g_boys_mu);
   if (device < 0 || device >= 64) return set_error(GBX_ERR_INVALID, "bad device %d", device);
+  // the quadrature kernel's table too is resolved here, before any stream capture
+  const double* rys = nullptr;
+  int s = rys_table(&rys);
+  if (s) return s;
   if (!g_boys_dev[device]) {
     std::vector<double> h((size_t)kBoysNGrid * (kBoysOrders + 1));
     boys_host_table(h.data());

@@ -36,6 +36,7 @@ constexpr int kStageBuffers = 3;                // host-output staging slabs in 
 constexpr size_t kStageBytes = 64ull << 20;     // target bytes of one staging slab
 
 int boys_table(int device, const double** out);
+int rys_table(const double** out);  // quadrature points and weights on the current device
 int compiled_lmax();
 
 // Diagonal blocks whose quartets run from the better-conditioned pair (quartet_transposed):
@@ -52,7 +53,7 @@ struct HostBlock {
   BlockDev dev;
   double avg_prims = 1.0;  // mean primitive quartets per shell quartet
   int team = 1;            // lanes per quartet (register kernel), set by heuristic or autotuner
-  int variant = 0;         // heavy classes with both kernels: 0 split, 1 line kernel
+  int variant = 0;         // heavy classes' kernel (EriLaunch::variant)
   int ctas_per_sm = 8;     // grid cap of the register kernel: resident-CTA multiples of the SMs
   long long j_computed = 0;  // quartets the last direct-J call computed in this block
 };

@@ -1,0 +1,541 @@
+// Quadrature kernel for heavy classes: a CTA of C::kW warps per contracted quartet.
+//
+// [e0|f0] of a primitive quartet is a sum over n = L/2 + 1 Rys points of Ix Iy Iz (plan and
+// tables: gen_rys.py), so the points of all primitive quartets of a contracted quartet form one
+// long contraction index k.  Per chunk of up to kRysKC points:
+//   points: thread k evaluates its point's abscissa and weight (piecewise polynomials of T) and
+//           writes the recursion coefficients P[.][k];
+//   tables: threads (axis, k) run the two-index recursion and write I[axis][(e, f)][k];
+//   sums:   the warps run the columns' matrix products X Y * Z over the chunk on the FP64 matrix
+//           instruction, sums in registers (C::gemm).
+// The tables have k innermost: a matrix operand is 8 table rows x 4 points.  After the last chunk
+// the sums go to shared memory ACC[e][f] once and
+// the whole CTA runs the tail: horizontal recursions, transforms, store / Schwarz maximum /
+// Coulomb contributions.
+//
+// What bounds it: shared-memory bandwidth (80 to 90 % of the LSU data pipe on (pd|sd), (pf|sf),
+// (df|sf), (pd|pd); FP64 pipe 45 to 55 %).  The matrix instruction is there for its operand reuse:
+// the same sums with a lane per column and FMAs read 8 shared values for every 9 FMAs and took 1.4
+// to 2 times longer.  Measured on the 20-atom chain's first 10 atoms (spherical, unique integrals,
+// blocks one after another), the line or split kernel before against this one: all heavy classes
+// 97.6 -> 17.9 ms; (pf|sf) 5.05 -> 0.89, (df|pf) 5.24 -> 0.50, (ff|ff) 2.03 -> 0.14, (pd|pd) 2.38
+// -> 0.32 ms (12.3 TF/s of algorithmic work, 36 % of the FP64 rate).  Error against 64-bit
+// reference values: tensors of the 60-molecule batch 2.0e-13 before, 2.8e-14 now.
+//
+// Mathematics: [e0|f0] as gbasis/integrals/_two_elec_int.py:293-547 defines it (the engine's other
+// kernels build the same values by the vertical and transfer recursions), :549-812 (horizontal
+// recursion, component norm), gbasis/base_four_symm.py:195-349 (norm_cont, spherical transform).
+#pragma once
+#include <algorithm>
+#include <atomic>
+
+#include "eri_kernels.cuh"  // gen::Sph, gen::cnorm
+#include "errors.h"
+#include "gbx_common.cuh"
+
+namespace gbx {
+
+constexpr int kRysKC = 32;           // quadrature points per chunk
+constexpr int kRysKS = kRysKC + 4;   // row stride of the tables: 4 rows x 4 points cover the banks
+constexpr int kRysDeg = 11;          // degree of the point polynomials (unit intervals of T)
+constexpr long long kRysMaxSmem = 227 * 1024;
+
+__host__ __device__ constexpr int rys_tmax(int n) {
+  return n == 3 ? 56 : n == 4 ? 60 : n == 5 ? 65 : n == 6 ? 70 : 76;
+}
+// Doubles before the n-point table.
+__host__ __device__ constexpr int rys_table_offset(int n) {
+  int o = 0;
+  for (int m = 3; m < n; ++m) o += (rys_tmax(m) * (kRysDeg + 1) + 1) * m * 2;
+  return o;
+}
+int rys_table(const double** out);
+
+__host__ __device__ constexpr int rys_tet(int k) { return k * (k + 1) * (k + 2) / 6; }
+// Components of total angular momentum lo..hi.
+__host__ __device__ constexpr int rys_ncomp(int lo, int hi) { return rys_tet(hi + 1) - rys_tet(lo); }
+
+// Abscissa (in t^2) and weight of point r of the N-point rule for exp(-T t^2) on [0, 1].
+template <int N>
+__device__ __forceinline__ double2 rys_point(double T, int r, const double* __restrict__ tab) {
+  constexpr int TM = rys_tmax(N);
+  if (T < (double)TM) {
+    const int i = (int)T;
+    const double u = fma(2.0, T - (double)i, -1.0);
+    const double2* __restrict__ c =
+        reinterpret_cast<const double2*>(tab) + (size_t)i * (kRysDeg + 1) * N + r;
+    double2 v = __ldg(c + kRysDeg * N);
+#pragma unroll
+    for (int d = kRysDeg - 1; d >= 0; --d) {
+      const double2 g = __ldg(c + d * N);
+      v.x = fma(v.x, u, g.x);
+      v.y = fma(v.y, u, g.y);
+    }
+    return v;
+  }
+  const double2 h = __ldg(reinterpret_cast<const double2*>(tab) + (size_t)TM * (kRysDeg + 1) * N + r);
+  const double q = rsqrt(T);
+  return make_double2(h.x * (q * q), h.y * q);
+}
+
+// Rows of the per-point coefficients.
+enum RysRow { kB00, kB10, kB01, kC0, kD0 = kC0 + 3, kWt = kD0 + 3, kRysRows };
+
+// One axis of one point: I(0,0) = scale, I(e+1,0) = C I(e,0) + e B10 I(e-1,0),
+// I(e,f+1) = D I(e,f) + f B01 I(e,f-1) + e B00 I(e-1,f), into out[(e * RF + f) * kRysKS].
+template <int NE1, int NF1, int RF>
+__device__ __forceinline__ void rys_axis(double C, double D, double B00, double B10, double B01,
+                                         double scale, double* __restrict__ out) {
+  double a0[NE1], a1[NE1];
+  a1[0] = scale;
+#pragma unroll
+  for (int e = 1; e < NE1; ++e)
+    a1[e] = e == 1 ? C * a1[0] : fma((double)(e - 1) * B10, a1[e - 2], C * a1[e - 1]);
+#pragma unroll
+  for (int e = 0; e < NE1; ++e) {
+    out[e * RF * kRysKS] = a1[e];
+    a0[e] = 0.0;
+  }
+#pragma unroll
+  for (int f = 1; f < NF1; ++f) {
+    double nw[NE1];
+#pragma unroll
+    for (int e = 0; e < NE1; ++e) {
+      double v = D * a1[e];
+      if (f > 1) v = fma((double)(f - 1) * B01, a0[e], v);
+      if (e > 0) v = fma((double)e * B00, a1[e - 1], v);
+      nw[e] = v;
+    }
+#pragma unroll
+    for (int e = 0; e < NE1; ++e) {
+      out[(e * RF + f) * kRysKS] = nw[e];
+      a0[e] = a1[e];
+      a1[e] = nw[e];
+    }
+  }
+}
+
+// FP64 matrix instruction m8n8k4: C[row][col] += sum_k A[row][k] B[k][col]; lane l holds A[l / 4]
+// [l % 4], B[l % 4][l / 4] and C[l / 4][2 (l % 4) + (0, 1)].
+__device__ __forceinline__ void rys_mma(double& c0, double& c1, double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+               : "+d"(c0), "+d"(c1)
+               : "d"(a), "d"(b));
+}
+
+// A table value at a byte offset.
+__device__ __forceinline__ double rys_ld(const char* t, unsigned off) {
+  return *reinterpret_cast<const double*>(t + off);
+}
+
+// A matrix instruction's two sums to their places in ACC (0xffff: not a target).
+__device__ __forceinline__ void rys_put(unsigned at, double c0, double c1, double* __restrict__ ACC) {
+  if ((at & 0xffffu) != 0xffffu) ACC[at & 0xffffu] = c0;
+  if ((at >> 16) != 0xffffu) ACC[at >> 16] = c1;
+}
+
+// Sizes of a class's kernel.
+template <class C>
+struct RysDims {
+  static constexpr int NE1 = C::LA + C::LB + 1, NF1 = C::LC + C::LD + 1;
+  static constexpr int NE = rys_ncomp(C::LA, C::LA + C::LB), NF = rys_ncomp(C::LC, C::LC + C::LD);
+  static constexpr int NFs = NF | 1;  // row stride of ACC (odd: lanes on consecutive rows)
+  static constexpr int NCA = ncart(C::LA), NCB = ncart(C::LB), NCC = ncart(C::LC), NCD = ncart(C::LD);
+  static constexpr int NAB = NCA * NCB, NKET = NCC * NCD;
+  static constexpr int HS = C::LD == 0 ? NFs : (NKET | 1);  // row stride of [e0|cd]
+  static constexpr int NT = 32 * C::kW;
+  // registers for 16 resident warps per SM where the sums leave room, else 12 or 8
+  static constexpr int kMinCtas = (C::kAcc <= 24 ? 16 : C::kAcc <= 36 ? 12 : 8) / C::kW;
+  static constexpr int RF = NF1 | 1;             // table rows per e
+  static constexpr int TS = NE1 * RF * kRysKS;   // one axis's table
+  // shared memory (doubles): ACC, overlaid after the ket recursion by the bra step's block of
+  // columns; then the tables and coefficients, overlaid by [e0|cd]
+  static constexpr int kAccSize = NE * NFs > 3 * NAB ? NE * NFs : 3 * NAB;
+  static constexpr int kAccEven = (kAccSize + 1) & ~1;
+  static constexpr int kTabSize = 3 * TS + kRysRows * kRysKS;
+  static constexpr int kHf = C::LD == 0 ? 0 : NE * HS;
+  static constexpr int kSmem = kAccEven + (kTabSize > kHf ? kTabSize : kHf);
+  // [e0|cd] of classes whose ket pair has no second angular momentum is ACC itself: the bra
+  // step's block then sits in the tables' place
+  static constexpr int kBlkSize = C::LD == 0 ? kSmem - kAccEven : kAccSize;
+};
+
+// Horizontal recursion onto a shell of angular momentum L for one component c of the first shell
+// (angular momentum L0): values [c + j], |j| <= L, read at in[index * stride] (components of total
+// L0.. in order), shifted along each axis in turn, in place:
+// (c, b) = sum_k binom(b, k) AB^(b-k) [c + k].  out: the ncart(L) components (c, b).
+template <int L0, int L>
+__device__ __forceinline__ void rys_hrr(const double* __restrict__ in, int stride, int c, double ABx,
+                                        double ABy, double ABz, double* __restrict__ out) {
+  const int u = (c >= 1) + (c >= 3) + (c >= 6);  // y + z of component c (at most 10 components)
+  const int zc = c - u * (u + 1) / 2;
+  double v[L + 1][L + 1][L + 1];
+#pragma unroll
+  for (int jx = 0; jx <= L; ++jx)
+#pragma unroll
+    for (int jy = 0; jy <= L - jx; ++jy)
+#pragma unroll
+      for (int jz = 0; jz <= L - jx - jy; ++jz) {
+        const int a = u + jy + jz;
+        v[jx][jy][jz] =
+            in[(rys_tet(L0 + jx + jy + jz) - rys_tet(L0) + a * (a + 1) / 2 + zc + jz) * stride];
+      }
+#pragma unroll
+  for (int jy = 0; jy <= L; ++jy)
+#pragma unroll
+    for (int jz = 0; jz <= L - jy; ++jz)
+#pragma unroll
+      for (int s = 1; s <= L - jy - jz; ++s)
+#pragma unroll
+        for (int j = L - jy - jz; j >= s; --j) v[j][jy][jz] = fma(ABx, v[j - 1][jy][jz], v[j][jy][jz]);
+#pragma unroll
+  for (int bx = 0; bx <= L; ++bx)
+#pragma unroll
+    for (int jz = 0; jz <= L - bx; ++jz)
+#pragma unroll
+      for (int s = 1; s <= L - bx - jz; ++s)
+#pragma unroll
+        for (int j = L - bx - jz; j >= s; --j) v[bx][j][jz] = fma(ABy, v[bx][j - 1][jz], v[bx][j][jz]);
+#pragma unroll
+  for (int bx = 0; bx <= L; ++bx)
+#pragma unroll
+    for (int by = 0; by <= L - bx; ++by)
+#pragma unroll
+      for (int s = 1; s <= L - bx - by; ++s)
+#pragma unroll
+        for (int j = L - bx - by; j >= s; --j) v[bx][by][j] = fma(ABz, v[bx][by][j - 1], v[bx][by][j]);
+  int k = 0;
+#pragma unroll
+  for (int bx = L; bx >= 0; --bx)
+#pragma unroll
+    for (int by = L - bx; by >= 0; --by) out[k++] = v[bx][by][L - bx - by];
+}
+
+struct RysArgs {
+  EriLaunch a;
+  const double* tab;  // rys_table()
+};
+
+// Per-quartet shell data in shared memory: A, B, C, D.
+struct RysShells {
+  double scl[4][kMaxCart];
+  int pos[4][kMaxCart];
+  int func[4], nint[4], nout[4];
+};
+
+template <int NW>
+__device__ __forceinline__ void rys_sync() {
+  if constexpr (NW == 1) __syncwarp();
+  else __syncthreads();
+}
+
+template <class C>
+__global__ void __launch_bounds__(32 * C::kW, RysDims<C>::kMinCtas) eri_rys(const RysArgs A) {
+  using D = RysDims<C>;
+  constexpr int N = C::kN, NT = D::NT, LA = C::LA, LB = C::LB, LC = C::LC, LD = C::LD;
+  extern __shared__ __align__(16) double smem[];
+  __shared__ RysShells S;
+  __shared__ long long s_next[2];
+  const EriLaunch& a = A.a;
+  const int tid = threadIdx.x, lane = tid & 31, wq = tid >> 5;
+  double* const ACC = smem;
+  double* const T = smem + D::kAccEven;
+  double* const PR = T + 3 * D::TS;
+  double* const HF = LD == 0 ? ACC : T;
+  double* const BLK = LD == 0 ? T : ACC;
+  const double* __restrict__ tab = A.tab + rys_table_offset(N);
+  const long long count = a.work_count ? (long long)(*a.work_count) : a.nwork;
+  const bool schwarz = a.mode == 1, coulomb = a.mode == 2;
+  double* const DCD = smem + D::kSmem;   // Coulomb mode: D[c][d] of the ket block,
+  double* const DAB = DCD + D::NKET;     // D[a][b] of the bra block,
+  double* const VAB = DAB + D::NAB;      // sum_cd (ab|cd) D[c][d]
+  long long w = blockIdx.x;
+  int turn = 0;
+  if (a.ticket) {  // quartets from the launch's counter; the next draw overlaps the quartet
+    if (tid == 0) s_next[0] = (long long)atomicAdd(a.ticket, 1ull);
+    rys_sync<C::kW>();
+    w = s_next[0];
+  }
+  while (w < count) {  // w is the same for all threads of the CTA
+    if (a.ticket && tid == 0) s_next[turn ^ 1] = (long long)atomicAdd(a.ticket, 1ull);
+    const int2 pq = a.work[a.reverse ? a.work_off + a.nwork - 1 - w : a.work_off + w];
+    const PairDev& P = a.pairs[pq.x];
+    const PairDev& Q = a.pairs[pq.y];
+    for (int i = tid; i < 4 * kMaxCart; i += NT) {
+      const int q = i / kMaxCart, c = i - q * kMaxCart;
+      const ShellDev& s = a.shells[q == 0 ? P.shA : q == 1 ? P.shB : q == 2 ? Q.shA : Q.shB];
+      S.scl[q][c] = s.scl[c];
+      S.pos[q][c] = s.pos[c];
+      if (c == 0) {
+        S.func[q] = s.func_off;
+        S.nout[q] = s.nout;
+        S.nint[q] = schwarz ? ncart(s.l) : internal_count(s);
+      }
+    }
+    const int nbp = P.nprim, nkp = Q.nprim, np = nbp * nkp;
+    const PrimPair* __restrict__ bprim = a.prims + P.prim_off;
+    const PrimPair* __restrict__ kprim = a.prims + Q.prim_off;
+    double acc[C::kAcc];
+#pragma unroll
+    for (int i = 0; i < C::kAcc; ++i) acc[i] = 0.0;
+    // points per primitive quartet: erfc(omega r)/r is 1/r minus erf(omega r)/r
+    const int kpp = a.potential == 2 ? 2 * N : N;
+    const int per_chunk = kRysKC / kpp;
+    for (int p0 = 0; p0 < np; p0 += per_chunk) {
+      const int kc = min(per_chunk, np - p0) * kpp, kcp = (kc + 3) & ~3;
+      // ---- points: by the last warp, whose share of the sums is the lightest
+      if (wq == C::kW - 1 && lane < kcp) {
+        const int k = lane;
+        double* const pr = PR + k;
+        if (k < kc) {
+          const int pi = k / kpp, r2 = k - pi * kpp, r = r2 < N ? r2 : r2 - N;
+          const int ip = (p0 + pi) / nkp, jq = p0 + pi - ip * nkp;
+          const PrimPair bp = bprim[ip], kp = kprim[jq];
+          const double rs = rsqrt(bp.zeta + kp.zeta), inv = rs * rs;
+          const double PQx = bp.Px - kp.Px, PQy = bp.Py - kp.Py, PQz = bp.Pz - kp.Pz;
+          const double rz = kp.zeta * inv, re = bp.zeta * inv;  // rho / zeta, rho / eta
+          const double rho = bp.zeta * rz;
+          double Tq = fmax(rho * fma(PQx, PQx, fma(PQy, PQy, PQz * PQz)), 0.0);
+          double pref = bp.C * kp.C * rs, sx = 1.0;
+          if (a.potential) {
+            // erf(omega r)/r: points and weights at s T, scaled by s and sqrt(s)
+            const bool att = a.potential == 1 || r2 >= N;
+            const double w2 = a.omega * a.omega;
+            if (att) {
+              sx = w2 / (w2 + rho);
+              Tq *= sx;
+              pref *= a.potential == 1 ? sqrt(sx) : -sqrt(sx);
+            }
+          }
+          const double2 xw = rys_point<N>(Tq, r, tab);
+          const double x = xw.x * sx;
+          const double o2z = 0.5 * bp.izeta, o2e = 0.5 * kp.izeta, xz = x * rz, xe = x * re;
+          pr[kB00 * kRysKS] = 0.5 * x * inv;
+          pr[kB10 * kRysKS] = fma(-xz, o2z, o2z);
+          pr[kB01 * kRysKS] = fma(-xe, o2e, o2e);
+          pr[kC0 * kRysKS] = fma(-xz, PQx, bp.Xx);
+          pr[(kC0 + 1) * kRysKS] = fma(-xz, PQy, bp.Xy);
+          pr[(kC0 + 2) * kRysKS] = fma(-xz, PQz, bp.Xz);
+          pr[kD0 * kRysKS] = fma(xe, PQx, kp.Xx);
+          pr[(kD0 + 1) * kRysKS] = fma(xe, PQy, kp.Xy);
+          pr[(kD0 + 2) * kRysKS] = fma(xe, PQz, kp.Xz);
+          pr[kWt * kRysKS] = pref * xw.y;
+        } else {
+#pragma unroll
+          for (int i = 0; i < kRysRows; ++i) pr[i * kRysKS] = 0.0;
+        }
+      }
+      rys_sync<C::kW>();  // points written; the previous chunk's tables are read
+      // ---- tables
+      for (int i = tid; i < 3 * kcp; i += NT) {
+        const int ax = i / kcp, k = i - ax * kcp;
+        const double* const pr = PR + k;
+        rys_axis<D::NE1, D::NF1, D::RF>(pr[(kC0 + ax) * kRysKS], pr[(kD0 + ax) * kRysKS], pr[kB00 * kRysKS],
+                                 pr[kB10 * kRysKS], pr[kB01 * kRysKS],
+                                 ax == 2 ? pr[kWt * kRysKS] : 1.0, T + ax * D::TS + k);
+      }
+      rys_sync<C::kW>();
+      // ---- sums
+      C::gemm(wq, lane, T, kcp, acc);
+    }
+    C::store(wq, lane, acc, ACC);
+    rys_sync<C::kW>();  // ACC complete, tables read
+    // ------------------------------------------------------------------------------ tail
+    const int nA = S.nint[0], nB = S.nint[1], nC = S.nint[2], nD = S.nint[3];
+    const int ncol = nC * nD;
+    if (coulomb) {
+      for (int i = tid; i < ncol; i += NT) {
+        const int uc = i / nD, ud = i - uc * nD;
+        DCD[i] = a.D[(S.func[2] + S.pos[2][uc]) * a.nbf + S.func[3] + S.pos[3][ud]] * S.scl[2][uc] *
+                 S.scl[3][ud];
+      }
+      for (int i = tid; i < nA * nB; i += NT) {
+        const int ua = i / nB, ub = i - ua * nB;
+        DAB[i] = a.D[(S.func[0] + S.pos[0][ua]) * a.nbf + S.func[1] + S.pos[1][ub]] * S.scl[0][ua] *
+                 S.scl[1][ub];
+        VAB[i] = 0.0;
+      }
+    }
+    // ket recursion and transform on D: tasks (row e, component c) -> HF[e][c][ud]
+    if constexpr (LD > 0) {
+      const double CDx = Q.ABx, CDy = Q.ABy, CDz = Q.ABz;
+      for (int t = tid; t < D::NE * D::NCC; t += NT) {
+        const int c = t / D::NE, e = t - c * D::NE;
+        double o[D::NCD];
+        rys_hrr<LC, LD>(ACC + e * D::NFs, 1, c, CDx, CDy, CDz, o);
+        if constexpr (LD >= 2) {
+          if (nD != D::NCD) {
+            double y[2 * LD + 1];
+            gen::Sph<LD>::apply(o, y);
+#pragma unroll
+            for (int i = 0; i < 2 * LD + 1; ++i) HF[e * D::HS + c * (2 * LD + 1) + i] = y[i];
+            continue;
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < D::NCD; ++i) HF[e * D::HS + c * D::NCD + i] = o[i];
+      }
+      rys_sync<C::kW>();
+    }
+    // transform on C, in place: tasks (row e, ud)
+    if constexpr (LC >= 2) {
+      if (nC != D::NCC) {
+        for (int t = tid; t < D::NE * nD; t += NT) {
+          const int ud = t / D::NE, e = t - ud * D::NE;
+          double* const row = HF + e * D::HS + ud;
+          double x[D::NCC], y[2 * LC + 1];
+#pragma unroll
+          for (int c = 0; c < D::NCC; ++c) x[c] = row[c * nD];
+          gen::Sph<LC>::apply(x, y);
+#pragma unroll
+          for (int c = 0; c < 2 * LC + 1; ++c) row[c * nD] = y[c];
+        }
+        rys_sync<C::kW>();
+      }
+    }
+    // bra recursion, transforms and output, a block of columns at a time
+    const double ABx = P.ABx, ABy = P.ABy, ABz = P.ABz;
+    const bool sphA = LA >= 2 && nA != D::NCA;
+    const bool block = sphA || coulomb;  // the columns' values meet in BLK[(a, ub)][column]
+    long long bbase, bcols;
+    block_dest(a, P, bbase, bcols);
+    const bool tr = quartet_transposed(P, Q);
+    const long long sbra = tr ? 1 : bcols, sket = tr ? bcols : 1;
+    const int rowlen = D::NCA * nB;
+    const int cap = block ? D::kBlkSize / rowlen : ncol;
+    const int cmax = block ? min(ncol, (cap & 1) ? cap : cap - 1) : ncol;  // odd row stride
+    const int CS = cmax | 1;
+    double mx = 0.0;
+    auto put = [&](int ua, int ub, int col, double v) {
+      const int uc = col / nD, ud = col - uc * nD;
+      const long long at = bbase +
+                           ((long long)P.fo + S.pos[0][ua] * S.nout[1] + S.pos[1][ub]) * sbra +
+                           ((long long)Q.fo + S.pos[2][uc] * S.nout[3] + S.pos[3][ud]) * sket;
+      out_store(a, at, v * (S.scl[0][ua] * S.scl[1][ub]) * (S.scl[2][uc] * S.scl[3][ud]));
+    };
+    for (int c0 = 0; c0 < ncol; c0 += cmax) {
+      const int cc = min(cmax, ncol - c0);
+      for (int t = tid; t < cc * D::NCA; t += NT) {
+        const int ca = t / cc, cl = t - ca * cc, col = c0 + cl;
+        double o[D::NCB];
+        rys_hrr<LA, LB>(HF + col, D::HS, ca, ABx, ABy, ABz, o);
+        if (schwarz) {
+          const int uc = col / nD, ud = col - uc * nD;
+          const double wcd = gen::cnorm<LC>(uc) * gen::cnorm<LD>(ud) * gen::cnorm<LA>(ca);
+#pragma unroll
+          for (int i = 0; i < D::NCB; ++i) mx = fmax(mx, fabs(o[i]) * (gen::cnorm<LB>(i) * wcd));
+          continue;
+        }
+        if constexpr (LB >= 2) {
+          if (nB != D::NCB) {
+            double y[2 * LB + 1];
+            gen::Sph<LB>::apply(o, y);
+#pragma unroll
+            for (int i = 0; i < 2 * LB + 1; ++i) o[i] = y[i];
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < D::NCB; ++i) {
+          if (i >= nB) break;
+          if (block) BLK[(ca * nB + i) * CS + cl] = o[i];
+          else put(ca, i, col, o[i]);
+        }
+      }
+      if (!block) continue;
+      rys_sync<C::kW>();
+      if constexpr (LA >= 2) {
+        if (sphA) {  // transform on A: tasks (ub, column), stored or put back in place
+          for (int t = tid; t < cc * nB; t += NT) {
+            const int ub = t / cc, cl = t - ub * cc;
+            double x[D::NCA], y[2 * LA + 1];
+#pragma unroll
+            for (int i = 0; i < D::NCA; ++i) x[i] = BLK[(i * nB + ub) * CS + cl];
+            gen::Sph<LA>::apply(x, y);
+#pragma unroll
+            for (int i = 0; i < 2 * LA + 1; ++i) {
+              if (coulomb) BLK[(i * nB + ub) * CS + cl] = y[i];
+              else put(i, ub, c0 + cl, y[i]);
+            }
+          }
+          rys_sync<C::kW>();
+        }
+      }
+      if (coulomb) {
+        // J[a][b] sums over the block's columns; J[c][d] of each column
+        const int nab = nA * nB;
+        for (int t = tid; t < nab + cc; t += NT) {
+          if (t < nab) {
+            double s = VAB[t];
+            for (int cl = 0; cl < cc; ++cl) s = fma(BLK[t * CS + cl], DCD[c0 + cl], s);
+            VAB[t] = s;
+          } else if (pq.x != pq.y) {
+            const int cl = t - nab, col = c0 + cl, uc = col / nD, ud = col - uc * nD;
+            double s = 0.0;
+            for (int i = 0; i < nab; ++i) s = fma(BLK[i * CS + cl], DAB[i], s);
+            s *= ((P.shA != P.shB) ? 2.0 : 1.0) * S.scl[2][uc] * S.scl[3][ud];
+            const long long fc = S.func[2] + S.pos[2][uc], fd = S.func[3] + S.pos[3][ud];
+            j_add(a, fc * a.nbf + fd, s);
+            if (Q.shA != Q.shB) j_add(a, fd * a.nbf + fc, s);
+          }
+        }
+        rys_sync<C::kW>();
+      }
+    }
+    if (schwarz) {
+      for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+      rys_sync<C::kW>();  // HF is read
+      if (lane == 0) smem[wq] = mx;
+      rys_sync<C::kW>();
+      if (tid == 0) {
+        for (int i = 1; i < C::kW; ++i) mx = fmax(mx, smem[i]);
+        a.qout[pq.x] = sqrt(mx);
+      }
+    }
+    if (coulomb) {
+      const double fk = (Q.shA != Q.shB) ? 2.0 : 1.0;
+      for (int i = tid; i < nA * nB; i += NT) {
+        const int ua = i / nB, ub = i - ua * nB;
+        const long long fa = S.func[0] + S.pos[0][ua], fb = S.func[1] + S.pos[1][ub];
+        const double s = VAB[i] * fk * S.scl[0][ua] * S.scl[1][ub];
+        j_add(a, fa * a.nbf + fb, s);
+        if (P.shA != P.shB) j_add(a, fb * a.nbf + fa, s);
+      }
+    }
+    rys_sync<C::kW>();  // shared memory free for the next quartet; the next draw is visible
+    turn ^= 1;
+    w = a.ticket ? s_next[turn] : w + gridDim.x;
+  }
+}
+
+template <class C>
+int launch_rys_t(const EriLaunch& a, cudaStream_t st) {
+  using D = RysDims<C>;
+  RysArgs A;
+  A.a = a;
+  int s = rys_table(&A.tab);
+  if (s) return s;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  const int cm = a.mode == 2 ? 1 : 0;
+  const int smem = (D::kSmem + (cm ? D::NKET + 2 * D::NAB : 0)) * (int)sizeof(double);
+  static_assert((D::kSmem + D::NKET + 2 * D::NAB) * 8 + 2048 <= kRysMaxSmem, "shared memory");
+  // CTAs the device keeps resident in this mode, found once per device and mode
+  static std::atomic<int> resident[64][2];
+  int r = dev >= 0 && dev < 64 ? resident[dev][cm].load() : 0;
+  if (!r) {
+    int per_sm = 0, nsm = 1;
+    const int most = (D::kSmem + D::NKET + 2 * D::NAB) * (int)sizeof(double);
+    s = cuda_status(cudaFuncSetAttribute(eri_rys<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, most),
+                    "eri_rys shared memory attribute");
+    if (s) return s;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, eri_rys<C>, D::NT, smem);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    r = std::max(1, per_sm) * nsm;
+    if (dev >= 0 && dev < 64) resident[dev][cm].store(r);
+  }
+  const int grid = (int)std::max<long long>(1, std::min<long long>(a.nwork, r));
+  eri_rys<C><<<grid, D::NT, smem, st>>>(A);
+  return cuda_status(cudaGetLastError(), "eri_rys launch");
+}
+
+}  // namespace gbx
