@@ -11,7 +11,7 @@ import threading
 
 import numpy as np
 
-from .contractions import is_shell
+from .contractions import GeneralizedContractionShell, is_shell
 
 __all__ = ["lib", "EngineError", "check", "pack_basis", "DeviceBasis", "EXPORTED_SYMBOLS",
            "library_path", "fp64_peak", "release_cached_memory"]
@@ -41,7 +41,7 @@ EXPORTED_SYMBOLS = (
     "gbx_basis_set_potential", "gbx_batch_run_mixed", "gbx_batch_mixed_counts", "gbx_boys_eval",
     "gbx_pipe_peak", "gbx_eri_coulomb_j_mixed", "gbx_set_block_config", "gbx_basis_set_streams",
     "gbx_batch_set_type_config", "gbx_mixed_counts", "gbx_batch_set_queue", "gbx_debug_bounds",
-    "gbx_basis_set_fp32_lists",
+    "gbx_basis_set_fp32_lists", "gbx_block_table",
 )
 
 
@@ -100,6 +100,7 @@ def lib():
             "gbx_num_blocks": [_P, ctypes.POINTER(_I)],
             "gbx_block_info": [_P, _I, _P, ctypes.POINTER(_I), ctypes.POINTER(_D),
                                ctypes.POINTER(_I64)],
+            "gbx_block_table": [_P, _I, _P, _P, _P, _P],
             "gbx_set_team": [_P, _I, _I],
             "gbx_block_times": [_P, _P, _I],
             "gbx_eri_full_mixed": [_P, _I, _D, _D, _P, _P],
@@ -180,6 +181,27 @@ def _canon_sph_labels(l):
 _P_LABEL = {(1, 0, 0): "c1", (0, 1, 0): "s1", (0, 0, 1): "c0"}
 
 
+# component norms sqrt((2x-1)!!(2y-1)!!(2z-1)!!) in canonical order, per l
+_SQRT_DFACT = tuple(np.sqrt(np.array([_dfact(2 * x - 1) * _dfact(2 * y - 1) * _dfact(2 * z - 1)
+                                      for x, y, z in _canon_cart(l)], dtype=float))
+                    for l in range(4))
+
+
+# positions 0..n-1 of n functions and the padding to MAX_CART slots, per n
+_IDENTITY = tuple(list(range(n)) + [-1] * (MAX_CART - n) for n in range(MAX_CART + 1))
+_ZEROS = tuple([0.0] * (MAX_CART - n) for n in range(MAX_CART + 1))
+
+
+def _default_orders(shell):
+    """Whether the shell has this package's own component orders (canonical, no signs): their
+    properties are the ones of :class:`GeneralizedContractionShell` itself."""
+    cls = type(shell)
+    return (getattr(cls, "angmom_components_cart", None)
+            is GeneralizedContractionShell.angmom_components_cart
+            and getattr(cls, "angmom_components_sph", None)
+            is GeneralizedContractionShell.angmom_components_sph)
+
+
 def _norm_cont(shell):
     coeffs = np.asarray(shell.coeffs)
     M = coeffs.shape[1] if coeffs.ndim == 2 else 1
@@ -187,9 +209,12 @@ def _norm_cont(shell):
     return np.asarray(shell.norm_cont, dtype=float).reshape(M, L)
 
 
+_COORD_NAMES = {"c": "cartesian", "p": "spherical"}
+
+
 def _coord_type(shell, override=None):
     ct = override if override is not None else shell.coord_type
-    ct = {"c": "cartesian", "p": "spherical"}.get(ct, ct)
+    ct = _COORD_NAMES.get(ct, ct)
     if ct not in ("cartesian", "spherical"):
         raise ValueError("Each entry of `coord_types` must be one of 'cartesian' or 'spherical'.")
     return ct
@@ -212,6 +237,28 @@ def pack_basis(shells, coord_types=None, raw=False):
         c = np.asarray(sh.coeffs, dtype=float)
         c = c[:, None] if c.ndim == 1 else c
         ct = "cartesian" if raw else _coord_type(sh, None if coord_types is None else coord_types[si])
+        if l < len(_SQRT_DFACT) and _default_orders(sh):
+            # the canonical orders: what the general code below finds, without the searches
+            n_c, M, spherical = len(_SQRT_DFACT[l]), c.shape[1], ct == "spherical"
+            nc = np.ones((M, n_c)) if raw else np.asarray(sh.norm_cont, dtype=float).reshape(M, n_c)
+            n_o = 2 * l + 1 if spherical else n_c
+            if spherical and not (np.abs(nc - nc[:, :1]) <= 1e-14 * np.abs(nc[:, :1])).all():
+                raise NotImplementedError(
+                    f"shell {si}: spherical transform with component-dependent norm_cont")
+            center, e_list = np.asarray(sh.coord, dtype=float).ravel().tolist(), e.tolist()
+            scale = (nc[:, :1] * np.ones(n_o) if spherical else nc / _SQRT_DFACT[l]).tolist()
+            for m, column in enumerate(c.T.tolist()):
+                ang.append(l)
+                npr.append(len(e_list))
+                cen += center
+                exps += e_list
+                coefs += column
+                nout.append(n_o)
+                sph.append(1 if spherical else 0)
+                pos.append(_IDENTITY[n_o])
+                scl.append(scale[m] + _ZEROS[n_o])
+                group.append(si)
+            continue
         cart = [tuple(int(v) for v in r) for r in np.asarray(sh.angmom_components_cart)]
         if sorted(cart) != sorted(_canon_cart(l)):
             raise ValueError(f"shell {si}: angmom_components_cart is not a permutation of the "
@@ -364,14 +411,11 @@ class DeviceBasis:
         """[(class (la, lb, lc, ld), team, mean primitive quartets, quartets)] per class block."""
         n = ctypes.c_int()
         check(lib().gbx_num_blocks(self.handle, ctypes.byref(n)))
-        out = []
-        for k in range(n.value):
-            c4 = np.zeros(4, dtype=np.int32)
-            t, ap, nq = ctypes.c_int(), ctypes.c_double(), ctypes.c_int64()
-            check(lib().gbx_block_info(self.handle, k, _ptr(c4), ctypes.byref(t), ctypes.byref(ap),
-                                       ctypes.byref(nq)))
-            out.append((tuple(int(v) for v in c4), t.value, ap.value, nq.value))
-        return out
+        c4, t = np.zeros((n.value, 4), dtype=np.int32), np.zeros(n.value, dtype=np.int32)
+        ap, nq = np.zeros(n.value), np.zeros(n.value, dtype=np.int64)
+        check(lib().gbx_block_table(self.handle, n.value, _ptr(c4), _ptr(t), _ptr(ap), _ptr(nq)))
+        return [(tuple(c), tt, a, q) for c, tt, a, q in
+                zip(c4.tolist(), t.tolist(), ap.tolist(), nq.tolist())]
 
     def set_team(self, k, team):
         check(lib().gbx_set_team(self.handle, int(k), int(team)), "gbx_set_team")

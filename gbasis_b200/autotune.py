@@ -22,6 +22,7 @@ creation).  gbasis has no counterpart: it evaluates one quartet at a time in Num
 """
 from __future__ import annotations
 
+import functools
 import json
 import math
 import os
@@ -55,8 +56,13 @@ def cache_path():
                           os.path.join(os.path.dirname(os.path.abspath(__file__)), "tuning.json"))
 
 
+@functools.lru_cache(maxsize=4096)
+def _bucket_key(cls4, bucket):
+    return "%d%d%d%d:%d" % (*cls4, bucket)
+
+
 def _key(cls4, avg_prims):
-    return "%d%d%d%d:%d" % (*cls4, int(round(math.log2(max(avg_prims, 1.0)))))
+    return _bucket_key(cls4, int(round(math.log2(max(avg_prims, 1.0)))))
 
 
 _loaded = {}  # path -> (modification time, table): read once per change of the file
@@ -81,6 +87,7 @@ def apply_cache(db, table=None):
     """Set the knobs of every block whose (class, primitive bucket) the cache knows, and the
     stream count; returns how many blocks changed."""
     table = _load() if table is None else table
+    configs = any(key.startswith(("v:", "c:")) for key in table)
     n = 0
     for k, (cls4, team, avg, _) in enumerate(db.blocks()):
         key = _key(cls4, avg)
@@ -88,6 +95,8 @@ def apply_cache(db, table=None):
         if t and t != team:
             db.set_team(k, int(t))
             n += 1
+        if not configs:
+            continue
         v, c = table.get("v:" + key), table.get("c:" + key)
         if v is not None or c is not None:
             db.set_block_config(k, int(v or 0), int(c or 8))

@@ -221,7 +221,8 @@ def electron_repulsion_integral_batch(molecules, notation="physicist", device=No
     if precision == "mixed":
         mixed = (MIXED_SKIP if mixed_skip is None else float(mixed_skip),
                  MIXED_FP32 if mixed_fp32 is None else float(mixed_fp32))
-    b = EriBatch(molecules, device=device)
+    # one run: launched as it is (capturing and instantiating a graph pays from the second run on)
+    b = EriBatch(molecules, device=device, graph=False)
     dev = torch.device("cuda", b.device)
     outs = [torch.empty((n,) * 4, dtype=torch.float64, device=dev) for n in b.nbf]
     b.run(outs, "chemist", stream=ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream),

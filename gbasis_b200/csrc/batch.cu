@@ -64,10 +64,8 @@ struct Batch {
   std::vector<ExpandArgs> h_exp;
   long long total_rows = 0, n_quartets = 0, compact_elems = 0;
   size_t max_row_bytes = 0;
+  std::unique_ptr<StreamSet> streams;  // kAuxStreams for the block types, one more to run on
   cudaStream_t exec = nullptr;
-  std::vector<cudaStream_t> aux;
-  std::vector<cudaEvent_t> join;
-  cudaEvent_t fork = nullptr, ev_in = nullptr, ev_out = nullptr;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t graph_exec = nullptr;
   bool use_graph = true;
@@ -75,7 +73,7 @@ struct Batch {
   // per-type timing (autotuner): types run one after another on the exec stream, eagerly
   bool profile = false;
   std::vector<cudaEvent_t> type_ev;
-  std::vector<void*> allocs;
+  std::vector<std::pair<void*, size_t>> allocs;
   // mixed-precision form: the FP64 work list and first merged pair of each molecule kept on
   // the host; per pair the bound of its output functions; per type, in d_work_mixed, the
   // FP64 quartets followed by the FP32 ones (quartets below the skip bound left out)
@@ -98,9 +96,10 @@ struct Batch {
   unsigned long long* d_fault = nullptr;  // debug builds: fault word of the bounds checks
 
   int alloc(void** p, size_t bytes, const char* what) {
-    if (bytes == 0) bytes = 16;
-    GBX_CUDA(cudaMalloc(p, bytes), what);
-    allocs.push_back(*p);
+    size_t got = 0;
+    const int s = block_alloc(device, p, bytes, &got, what);
+    if (s) return s;
+    allocs.push_back({*p, got});
     return GBX_OK;
   }
   template <typename T>
@@ -118,15 +117,46 @@ struct Batch {
     if (graph) cudaGraphDestroy(graph);
     if (graph_exec_m) cudaGraphExecDestroy(graph_exec_m);
     if (graph_m) cudaGraphDestroy(graph_m);
-    for (void* p : allocs) cudaFree(p);
-    for (cudaStream_t s : aux) cudaStreamDestroy(s);
-    for (cudaEvent_t e : join) cudaEventDestroy(e);
+    // blocks and streams are given back once nothing queued on the device can still use them
+    const bool idle = cudaDeviceSynchronize() == cudaSuccess;
+    for (auto& a : allocs) {
+      if (idle) block_give(device, a.first, a.second);
+      else cudaFree(a.first);
+    }
+    streams_give(std::move(streams), idle);
     for (cudaEvent_t e : type_ev) cudaEventDestroy(e);
-    if (fork) cudaEventDestroy(fork);
-    if (ev_in) cudaEventDestroy(ev_in);
-    if (ev_out) cudaEventDestroy(ev_out);
-    if (exec) cudaStreamDestroy(exec);
     if (prev >= 0) cudaSetDevice(prev);
+  }
+};
+
+// Host tables that go to the device in one block and one copy (a batch of small molecules has over
+// a hundred of them: two per block type besides the merged arrays).
+struct UploadSet {
+  struct Item {
+    void** d;
+    const void* h;
+    size_t bytes;
+  };
+  std::vector<Item> items;
+  template <typename T>
+  void add(T** d, const std::vector<T>& h) {
+    items.push_back({(void**)d, h.data(), h.size() * sizeof(T)});
+  }
+  int run(Batch& Bt) {
+    size_t total = 0;
+    for (const Item& t : items) total += (std::max<size_t>(t.bytes, 1) + 255) & ~(size_t)255;
+    unsigned char* block = nullptr;
+    int s = Bt.alloc((void**)&block, total, "cudaMalloc(batch tables)");
+    if (s) return s;
+    std::unique_ptr<unsigned char[]> host(new unsigned char[total]);
+    size_t at = 0;
+    for (const Item& t : items) {
+      *t.d = block + at;
+      if (t.bytes) memcpy(host.get() + at, t.h, t.bytes);
+      at += (std::max<size_t>(t.bytes, 1) + 255) & ~(size_t)255;
+    }
+    GBX_CUDA(cudaMemcpy(block, host.get(), total, cudaMemcpyHostToDevice), "upload batch tables");
+    return GBX_OK;
   }
 };
 
@@ -245,10 +275,11 @@ static int build_batch(Batch& Bt, int n_mol, const int* mol_nshells, const int* 
   // device arrays
   DeviceGuardLite g(Bt.device);
   int s;
-  if ((s = Bt.upload(&Bt.d_shells, shells, "upload batch shells"))) return s;
-  if ((s = Bt.upload(&Bt.d_pairs, pairs, "upload batch pairs"))) return s;
-  if ((s = Bt.upload(&Bt.d_exps, hexps, "upload batch exponents"))) return s;
-  if ((s = Bt.upload(&Bt.d_coefs, hcoefs, "upload batch coefficients"))) return s;
+  UploadSet up;
+  up.add(&Bt.d_shells, shells);
+  up.add(&Bt.d_pairs, pairs);
+  up.add(&Bt.d_exps, hexps);
+  up.add(&Bt.d_coefs, hcoefs);
   if ((s = Bt.upload(&Bt.d_work, work, "upload batch work list"))) return s;
   Bt.h_work = std::move(work);
   Bt.pair_off = pair_off;
@@ -256,13 +287,10 @@ static int build_batch(Batch& Bt, int n_mol, const int* mol_nshells, const int* 
                     "cudaMalloc(batch primitive pairs)")))
     return s;
   const int np = (int)pairs.size();
-  pair_precompute<<<(np + 127) / 128, 128>>>(Bt.d_pairs, np, Bt.d_shells, Bt.d_exps, Bt.d_coefs,
-                                             Bt.d_prims);
-  GBX_CUDA(cudaGetLastError(), "pair_precompute launch");
   if ((s = boys_table(Bt.device, &Bt.d_boys))) return s;
   for (size_t k = 0; k < Bt.types.size(); ++k) {
-    if ((s = Bt.upload(&Bt.types[k].d_base, tbase[k], "upload batch block bases"))) return s;
-    if ((s = Bt.upload(&Bt.types[k].d_ncols, tcols[k], "upload batch block columns"))) return s;
+    up.add(&Bt.types[k].d_base, tbase[k]);
+    up.add(&Bt.types[k].d_ncols, tcols[k]);
   }
   if ((s = Bt.alloc((void**)&Bt.d_compact, (size_t)Bt.compact_elems * sizeof(double),
                     "cudaMalloc(batch compact store)")))
@@ -287,12 +315,16 @@ static int build_batch(Batch& Bt, int n_mol, const int* mol_nshells, const int* 
     Bt.max_row_bytes = std::max(Bt.max_row_bytes, (size_t)npf * sizeof(double));
   }
   Bt.total_rows = row_first[n_mol];
-  if ((s = Bt.upload(&Bt.d_gtab, gtab, "upload batch gtab"))) return s;
-  if ((s = Bt.upload(&Bt.d_rowinfo, rowinfo, "upload batch rowinfo"))) return s;
-  if ((s = Bt.upload(&Bt.d_blocks, blocks, "upload batch block tables"))) return s;
-  if ((s = Bt.upload(&Bt.d_row_first, row_first, "upload batch row offsets"))) return s;
+  up.add(&Bt.d_gtab, gtab);
+  up.add(&Bt.d_rowinfo, rowinfo);
+  up.add(&Bt.d_blocks, blocks);
+  up.add(&Bt.d_row_first, row_first);
+  if ((s = up.run(Bt))) return s;
+  pair_precompute<<<(np + 127) / 128, 128>>>(Bt.d_pairs, np, Bt.d_shells, Bt.d_exps, Bt.d_coefs,
+                                             Bt.d_prims);
+  GBX_CUDA(cudaGetLastError(), "pair_precompute launch");
   if ((s = alloc_fault_word(&Bt.d_fault))) return s;
-  if (Bt.d_fault) Bt.allocs.push_back(Bt.d_fault);
+  if (Bt.d_fault) Bt.allocs.push_back({Bt.d_fault, sizeof(unsigned long long)});
   Bt.h_exp.resize(n_mol);
   for (int m = 0; m < n_mol; ++m) {
     const Basis& B = *Bt.mols[m];
@@ -318,17 +350,10 @@ static int build_batch(Batch& Bt, int n_mol, const int* mol_nshells, const int* 
   if ((s = Bt.alloc((void**)&Bt.d_tickets, 2 * Bt.types.size() * sizeof(unsigned long long),
                     "cudaMalloc(batch work counters)")))
     return s;
-  GBX_CUDA(cudaStreamCreateWithFlags(&Bt.exec, cudaStreamNonBlocking), "create stream");
-  Bt.aux.resize(kAuxStreams);
-  Bt.join.resize(kAuxStreams);
-  for (int j = 0; j < kAuxStreams; ++j) {
-    GBX_CUDA(cudaStreamCreateWithFlags(&Bt.aux[j], cudaStreamNonBlocking), "create stream");
-    GBX_CUDA(cudaEventCreateWithFlags(&Bt.join[j], cudaEventDisableTiming), "create event");
-  }
-  GBX_CUDA(cudaEventCreateWithFlags(&Bt.fork, cudaEventDisableTiming), "create event");
-  GBX_CUDA(cudaEventCreateWithFlags(&Bt.ev_in, cudaEventDisableTiming), "create event");
-  GBX_CUDA(cudaEventCreateWithFlags(&Bt.ev_out, cudaEventDisableTiming), "create event");
-  GBX_CUDA(cudaDeviceSynchronize(), "batch upload");
+  if ((s = streams_take(Bt.device, &Bt.streams))) return s;
+  if ((s = Bt.streams->ensure_aux(kAuxStreams + 1))) return s;
+  Bt.exec = Bt.streams->aux[kAuxStreams];
+  GBX_CUDA(cudaStreamSynchronize(nullptr), "batch upload");
   return GBX_OK;
 }
 
@@ -357,14 +382,17 @@ static int batch_mixed_bounds(Batch& Bt) {
   if ((long long)diag.size() != np)
     return set_error(GBX_ERR_INVALID, "batch pair classes cover %lld of %lld pairs",
                      (long long)diag.size(), np);
-  int2* d_diag = nullptr;
-  double* d_q = nullptr;
-  GBX_CUDA(cudaMalloc(&d_diag, std::max<size_t>(diag.size(), 1) * sizeof(int2)),
-           "cudaMalloc(batch diagonal quartets)");
-  cudaError_t e = cudaMalloc(&d_q, std::max<long long>(np, 1) * sizeof(double));
-  if (e == cudaSuccess)
-    e = cudaMemcpy(d_diag, diag.data(), diag.size() * sizeof(int2), cudaMemcpyHostToDevice);
-  int s = cuda_status(e, "batch mixed-form bounds setup");
+  // quartets and bounds in one block of the cache
+  const size_t q_at = (std::max<size_t>(diag.size(), 1) * sizeof(int2) + 255) & ~(size_t)255;
+  unsigned char* tmp = nullptr;
+  size_t got = 0;
+  int s = block_alloc(Bt.device, (void**)&tmp, q_at + std::max<long long>(np, 1) * sizeof(double),
+                      &got, "cudaMalloc(batch diagonal quartets)");
+  if (s) return s;
+  int2* d_diag = reinterpret_cast<int2*>(tmp);
+  double* d_q = reinterpret_cast<double*>(tmp + q_at);
+  cudaError_t e = cudaMemcpy(d_diag, diag.data(), diag.size() * sizeof(int2), cudaMemcpyHostToDevice);
+  s = cuda_status(e, "batch mixed-form bounds setup");
   const int nsm = num_sms_of(Bt.device);
   for (int c = 0; c < kNumPairClasses && !s; ++c) {
     const long long n = first[c + 1] - first[c];
@@ -408,8 +436,8 @@ static int batch_mixed_bounds(Batch& Bt) {
                                cudaMemcpyDeviceToHost), "download batch bounds");
     if (s) Bt.h_qmixed.clear();
   }
-  cudaFree(d_diag);
-  if (d_q) cudaFree(d_q);
+  if (e == cudaSuccess) block_give(Bt.device, tmp, got);  // the stream is idle
+  else cudaFree(tmp);
   return s;
 }
 
@@ -550,15 +578,16 @@ static int enqueue_batch(Batch& Bt, cudaStream_t st, bool mixed = false) {
   if (tickets)
     GBX_CUDA(cudaMemsetAsync(Bt.d_tickets, 0, 2 * Bt.types.size() * sizeof(unsigned long long), st),
              "clear batch work counters");
-  GBX_CUDA(cudaEventRecord(Bt.fork, st), "fork");
-  for (cudaStream_t a : Bt.aux) GBX_CUDA(cudaStreamWaitEvent(a, Bt.fork, 0), "fork wait");
+  StreamSet& S = *Bt.streams;
+  GBX_CUDA(cudaEventRecord(S.fork, st), "fork");
+  for (int j = 0; j < kAuxStreams; ++j) GBX_CUDA(cudaStreamWaitEvent(S.aux[j], S.fork, 0), "fork wait");
   for (size_t i = 0; i < Bt.order.size(); ++i) {
     const int k = Bt.order[i];
     const BatchType& T = Bt.types[k];
     if (Bt.profile) GBX_CUDA(cudaEventRecord(Bt.type_ev[i], st), "type event");
     EriLaunch a = type_launch(Bt, k);
     a.ticket = tickets ? Bt.d_tickets + 2 * k : nullptr;
-    cudaStream_t ts = Bt.profile ? st : Bt.aux[i % Bt.aux.size()];
+    cudaStream_t ts = Bt.profile ? st : S.aux[i % kAuxStreams];
     if (mixed) {
       a.work = Bt.d_work_mixed;
       a.work_off = Bt.mix_off[k];
@@ -584,9 +613,9 @@ static int enqueue_batch(Batch& Bt, cudaStream_t st, bool mixed = false) {
     }
   }
   if (Bt.profile) GBX_CUDA(cudaEventRecord(Bt.type_ev[Bt.order.size()], st), "type event");
-  for (size_t j = 0; j < Bt.aux.size(); ++j) {
-    GBX_CUDA(cudaEventRecord(Bt.join[j], Bt.aux[j]), "join");
-    GBX_CUDA(cudaStreamWaitEvent(st, Bt.join[j], 0), "join wait");
+  for (int j = 0; j < kAuxStreams; ++j) {
+    GBX_CUDA(cudaEventRecord(S.join[j], S.aux[j]), "join");
+    GBX_CUDA(cudaStreamWaitEvent(st, S.join[j], 0), "join wait");
   }
   return launch_expand_batch(Bt.device, Bt.d_exp, Bt.d_row_first, Bt.nmol, Bt.total_rows,
                              Bt.max_row_bytes, st);
@@ -605,8 +634,8 @@ static int run_batch(Batch& Bt, int notation, double* const* outs, cudaStream_t 
     Bt.h_exp[m].out_lo = outs[m];
     Bt.h_exp[m].notation = notation;
   }
-  GBX_CUDA(cudaEventRecord(Bt.ev_in, caller), "record caller");
-  GBX_CUDA(cudaStreamWaitEvent(Bt.exec, Bt.ev_in, 0), "wait caller");
+  GBX_CUDA(cudaEventRecord(Bt.streams->in, caller), "record caller");
+  GBX_CUDA(cudaStreamWaitEvent(Bt.exec, Bt.streams->in, 0), "wait caller");
   if (changed) {
     Bt.exp_dirty = true;  // until the device table holds these outputs
     GBX_CUDA(cudaMemcpyAsync(Bt.d_exp, Bt.h_exp.data(), Bt.nmol * sizeof(ExpandArgs),
@@ -641,8 +670,8 @@ static int run_batch(Batch& Bt, int notation, double* const* outs, cudaStream_t 
     const int s = enqueue_batch(Bt, Bt.exec, mx);
     if (s) return s;
   }
-  GBX_CUDA(cudaEventRecord(Bt.ev_out, Bt.exec), "record batch");
-  GBX_CUDA(cudaStreamWaitEvent(caller, Bt.ev_out, 0), "caller wait");
+  GBX_CUDA(cudaEventRecord(Bt.streams->out, Bt.exec), "record batch");
+  GBX_CUDA(cudaStreamWaitEvent(caller, Bt.streams->out, 0), "caller wait");
   return GBX_OK;
 }
 

@@ -595,79 +595,64 @@ int upload_basis(Basis& B) {
   const int n = (int)B.shells.size();
   const int np = (int)B.pairs.size();
   int s;
-  if ((s = B.alloc((void**)&B.d_shells, n * sizeof(ShellDev), "cudaMalloc(shells)"))) return s;
-  if ((s = B.alloc((void**)&B.d_pairs, np * sizeof(PairDev), "cudaMalloc(pairs)"))) return s;
-  if ((s = B.alloc((void**)&B.d_prims, B.n_prim_pairs * sizeof(PrimPair), "cudaMalloc(prims)")))
-    return s;
-  if ((s = B.alloc((void**)&B.d_exps, B.h_exps.size() * sizeof(double), "cudaMalloc(exps)")))
-    return s;
-  if ((s = B.alloc((void**)&B.d_coefs, B.h_coefs.size() * sizeof(double), "cudaMalloc(coefs)")))
-    return s;
-  if ((s = B.alloc((void**)&B.d_pair_of, (size_t)n * n * sizeof(int), "cudaMalloc(pair_of)")))
-    return s;
-  GBX_CUDA(cudaMemcpy(B.d_shells, B.shells.data(), n * sizeof(ShellDev), cudaMemcpyHostToDevice),
-           "upload shells");
-  GBX_CUDA(cudaMemcpy(B.d_pairs, B.pairs.data(), np * sizeof(PairDev), cudaMemcpyHostToDevice),
-           "upload pairs");
-  GBX_CUDA(cudaMemcpy(B.d_exps, B.h_exps.data(), B.h_exps.size() * sizeof(double),
-                      cudaMemcpyHostToDevice), "upload exps");
-  GBX_CUDA(cudaMemcpy(B.d_coefs, B.h_coefs.data(), B.h_coefs.size() * sizeof(double),
-                      cudaMemcpyHostToDevice), "upload coefs");
-  GBX_CUDA(cudaMemcpy(B.d_pair_of, B.pair_of.data(), (size_t)n * n * sizeof(int),
-                      cudaMemcpyHostToDevice), "upload pair_of");
-  pair_precompute<<<(np + 127) / 128, 128>>>(B.d_pairs, np, B.d_shells, B.d_exps, B.d_coefs,
-                                             B.d_prims);
-  GBX_CUDA(cudaGetLastError(), "pair_precompute launch");
-
-  // function tables
+  const int nblk = (int)B.blocks.size();
   std::vector<int> fsh(B.nbf), fcomp(B.nbf);
   for (int sh = 0; sh < n; ++sh)
     for (int c = 0; c < B.shells[sh].nout; ++c) {
       fsh[B.shells[sh].func_off + c] = sh;
       fcomp[B.shells[sh].func_off + c] = c;
     }
-  if ((s = B.alloc((void**)&B.d_func_shell, B.nbf * sizeof(int), "cudaMalloc(fsh)"))) return s;
-  if ((s = B.alloc((void**)&B.d_func_comp, B.nbf * sizeof(int), "cudaMalloc(fcomp)"))) return s;
-  GBX_CUDA(cudaMemcpy(B.d_func_shell, fsh.data(), B.nbf * sizeof(int), cudaMemcpyHostToDevice),
-           "upload fsh");
-  GBX_CUDA(cudaMemcpy(B.d_func_comp, fcomp.data(), B.nbf * sizeof(int), cudaMemcpyHostToDevice),
-           "upload fcomp");
-  if ((s = B.alloc((void**)&B.d_blocks, B.block_table.size() * sizeof(BlockDev),
-                   "cudaMalloc(blocks)")))
-    return s;
-  GBX_CUDA(cudaMemcpy(B.d_blocks, B.block_table.data(), B.block_table.size() * sizeof(BlockDev),
-                      cudaMemcpyHostToDevice), "upload blocks");
-
-  const int nblk = (int)B.blocks.size();
-  if ((s = B.alloc((void**)&B.d_counts, (nblk + 4) * sizeof(int), "cudaMalloc(counts)"))) return s;
-  if ((s = B.alloc((void**)&B.d_pinfo, np * sizeof(int4), "cudaMalloc(pinfo)"))) return s;
   std::vector<int4> pinfo(np);
   for (int p = 0; p < np; ++p)
     pinfo[p] = make_int4(B.pairs[p].cls, B.pairs[p].local, B.pairs[p].fo, B.pairs[p].nB);
-  GBX_CUDA(cudaMemcpy(B.d_pinfo, pinfo.data(), np * sizeof(int4), cudaMemcpyHostToDevice),
-           "upload pinfo");
-  if ((s = B.alloc((void**)&B.d_ftab, B.h_ftab.size() * sizeof(long long), "cudaMalloc(ftab)")))
-    return s;
-  GBX_CUDA(cudaMemcpy(B.d_ftab, B.h_ftab.data(), B.h_ftab.size() * sizeof(long long),
-                      cudaMemcpyHostToDevice), "upload ftab");
-  if ((s = B.alloc((void**)&B.d_gtab, B.h_gtab.size() * sizeof(int), "cudaMalloc(gtab)")))
-    return s;
-  GBX_CUDA(cudaMemcpy(B.d_gtab, B.h_gtab.data(), B.h_gtab.size() * sizeof(int),
-                      cudaMemcpyHostToDevice), "upload gtab");
-  if ((s = B.alloc((void**)&B.d_rowinfo, B.h_rowinfo.size() * sizeof(int4),
-                   "cudaMalloc(rowinfo)")))
-    return s;
-  GBX_CUDA(cudaMemcpy(B.d_rowinfo, B.h_rowinfo.data(), B.h_rowinfo.size() * sizeof(int4),
-                      cudaMemcpyHostToDevice), "upload rowinfo");
-  if ((s = B.alloc((void**)&B.d_q, np * sizeof(double), "cudaMalloc(q)"))) return s;
-  if ((s = B.alloc((void**)&B.d_qscreen, np * sizeof(double), "cudaMalloc(qscreen)"))) return s;
+  // one device block and one copy for all host tables (12 allocations and copies took most of the
+  // creation of a small basis), and one block for what the device writes
+  struct Table {
+    void** d;
+    const void* h;
+    size_t bytes, at;
+  };
+  std::vector<Table> tables = {
+      {(void**)&B.d_shells, B.shells.data(), n * sizeof(ShellDev), 0},
+      {(void**)&B.d_pairs, B.pairs.data(), np * sizeof(PairDev), 0},
+      {(void**)&B.d_exps, B.h_exps.data(), B.h_exps.size() * sizeof(double), 0},
+      {(void**)&B.d_coefs, B.h_coefs.data(), B.h_coefs.size() * sizeof(double), 0},
+      {(void**)&B.d_pair_of, B.pair_of.data(), (size_t)n * n * sizeof(int), 0},
+      {(void**)&B.d_func_shell, fsh.data(), B.nbf * sizeof(int), 0},
+      {(void**)&B.d_func_comp, fcomp.data(), B.nbf * sizeof(int), 0},
+      {(void**)&B.d_blocks, B.block_table.data(), B.block_table.size() * sizeof(BlockDev), 0},
+      {(void**)&B.d_pinfo, pinfo.data(), np * sizeof(int4), 0},
+      {(void**)&B.d_ftab, B.h_ftab.data(), B.h_ftab.size() * sizeof(long long), 0},
+      {(void**)&B.d_gtab, B.h_gtab.data(), B.h_gtab.size() * sizeof(int), 0},
+      {(void**)&B.d_rowinfo, B.h_rowinfo.data(), B.h_rowinfo.size() * sizeof(int4), 0},
+      {(void**)&B.d_prims, nullptr, B.n_prim_pairs * sizeof(PrimPair), 0},
+      {(void**)&B.d_counts, nullptr, (nblk + 4) * sizeof(int), 0},
+      {(void**)&B.d_q, nullptr, np * sizeof(double), 0},
+      {(void**)&B.d_qscreen, nullptr, np * sizeof(double), 0}};
+  size_t total = 0, upload = 0;
+  for (Table& t : tables) {
+    t.at = total;
+    total += (std::max<size_t>(t.bytes, 1) + 255) & ~(size_t)255;
+    if (t.h) upload = total;
+  }
+  unsigned char* block = nullptr;
+  if ((s = B.alloc((void**)&block, total, "cudaMalloc(basis tables)"))) return s;
+  std::unique_ptr<unsigned char[]> host(new unsigned char[upload]);
+  for (const Table& t : tables) {
+    *t.d = block + t.at;
+    if (t.h && t.bytes) std::memcpy(host.get() + t.at, t.h, t.bytes);
+  }
+  GBX_CUDA(cudaMemcpy(block, host.get(), upload, cudaMemcpyHostToDevice), "upload basis tables");
+  pair_precompute<<<(np + 127) / 128, 128>>>(B.d_pairs, np, B.d_shells, B.d_exps, B.d_coefs,
+                                             B.d_prims);
+  GBX_CUDA(cudaGetLastError(), "pair_precompute launch");
   if ((s = boys_table(B.device, &B.d_boys))) return s;
 #if GBX_DEBUG_BOUNDS
   if ((s = B.alloc((void**)&B.d_fault, sizeof(unsigned long long), "cudaMalloc(fault word)")))
     return s;
   GBX_CUDA(cudaMemset(B.d_fault, 0, sizeof(unsigned long long)), "clear fault word");
 #endif
-  GBX_CUDA(cudaDeviceSynchronize(), "basis upload");
+  GBX_CUDA(cudaStreamSynchronize(nullptr), "basis upload");
   return GBX_OK;
 }
 
@@ -683,7 +668,8 @@ static int ensure_full_work(Basis& B) {
   if (B.d_work) return GBX_OK;
   int s;
   const int nblk = (int)B.blocks.size();
-  if ((s = B.alloc((void**)&B.d_work, (size_t)B.n_quartets * sizeof(int2), "cudaMalloc(work)")))
+  int2* work = nullptr;
+  if ((s = B.alloc((void**)&work, (size_t)B.n_quartets * sizeof(int2), "cudaMalloc(work)")))
     return s;
   std::vector<BuildBlock> bb(nblk);
   std::vector<int2> cmap;
@@ -698,15 +684,17 @@ static int ensure_full_work(Basis& B) {
                        h.ncand);
   }
   B.n_cta_build = (int)cmap.size();
-  void* dbb = nullptr;
-  if ((s = B.alloc(&dbb, nblk * sizeof(BuildBlock), "cudaMalloc(build blocks)"))) return s;
-  if ((s = B.alloc((void**)&B.d_cta_map, cmap.size() * sizeof(int2), "cudaMalloc(cta map)")))
-    return s;
-  GBX_CUDA(cudaMemcpy(dbb, bb.data(), nblk * sizeof(BuildBlock), cudaMemcpyHostToDevice),
-           "upload build blocks");
-  GBX_CUDA(cudaMemcpy(B.d_cta_map, cmap.data(), cmap.size() * sizeof(int2), cudaMemcpyHostToDevice),
-           "upload cta map");
-  B.d_build_blocks = dbb;
+  const size_t at = (nblk * sizeof(BuildBlock) + 255) & ~(size_t)255;
+  const size_t bytes = at + cmap.size() * sizeof(int2);
+  unsigned char* block = nullptr;
+  if ((s = B.alloc((void**)&block, bytes, "cudaMalloc(build map)"))) return s;
+  std::unique_ptr<unsigned char[]> host(new unsigned char[bytes]);
+  std::memcpy(host.get(), bb.data(), nblk * sizeof(BuildBlock));
+  std::memcpy(host.get() + at, cmap.data(), cmap.size() * sizeof(int2));
+  GBX_CUDA(cudaMemcpy(block, host.get(), bytes, cudaMemcpyHostToDevice), "upload build map");
+  B.d_build_blocks = block;
+  B.d_cta_map = reinterpret_cast<int2*>(block + at);
+  B.d_work = work;  // set last: it marks the map as made
   return GBX_OK;
 }
 
@@ -762,9 +750,13 @@ int ensure_schwarz(Basis& B, cudaStream_t st) {
   std::vector<int2> diag(np);
   for (int p = 0; p < np; ++p) diag[p] = make_int2(p, p);
   int2* d_diag = nullptr;
-  GBX_CUDA(cudaMalloc(&d_diag, np * sizeof(int2)), "cudaMalloc(schwarz work)");
-  GBX_CUDA(cudaMemcpyAsync(d_diag, diag.data(), np * sizeof(int2), cudaMemcpyHostToDevice, st),
-           "upload schwarz work");
+  size_t got = 0;
+  int s0 = block_alloc(B.device, (void**)&d_diag, np * sizeof(int2), &got, "cudaMalloc(schwarz work)");
+  if (s0) return s0;
+  const cudaError_t e0 =
+      cudaMemcpyAsync(d_diag, diag.data(), np * sizeof(int2), cudaMemcpyHostToDevice, st);
+  if (e0 != cudaSuccess) cudaFree(d_diag);
+  GBX_CUDA(e0, "upload schwarz work");
   const int nsm = num_sms(B.device);
   for (int c = 0; c < kNumPairClasses; ++c) {
     if (B.class_count[c] == 0) continue;
@@ -786,7 +778,8 @@ int ensure_schwarz(Basis& B, cudaStream_t st) {
   std::vector<double> q(np);
   cudaError_t e1 = cudaMemcpyAsync(q.data(), B.d_q, np * sizeof(double), cudaMemcpyDeviceToHost, st);
   cudaError_t e2 = cudaStreamSynchronize(st);
-  cudaFree(d_diag);
+  if (e2 == cudaSuccess) block_give(B.device, d_diag, got);  // the stream is idle
+  else cudaFree(d_diag);
   GBX_CUDA(e1, "download schwarz bounds");
   GBX_CUDA(e2, "schwarz bounds");
   // bound of the original (generalized) shell pair: max over its segmented pairs
@@ -889,7 +882,8 @@ static int ensure_mixed_bounds(Basis& B, cudaStream_t st) {
   const size_t bytes = np * (sizeof(PairDev) + sizeof(int2) + 2 * sizeof(long long)) +
                        (size_t)off[np] * sizeof(double);
   unsigned char* tmp = nullptr;
-  GBX_CUDA(cudaMalloc(&tmp, bytes), "cudaMalloc(diagonal quartets)");
+  size_t got = 0;
+  if ((s = block_alloc(B.device, (void**)&tmp, bytes, &got, "cudaMalloc(diagonal quartets)"))) return s;
   PairDev* d_tp = reinterpret_cast<PairDev*>(tmp);
   int2* d_diag = reinterpret_cast<int2*>(d_tp + np);
   long long* d_off = reinterpret_cast<long long*>(d_diag + np);
@@ -926,7 +920,8 @@ static int ensure_mixed_bounds(Basis& B, cudaStream_t st) {
     e = cudaGetLastError();
   }
   const cudaError_t e2 = cudaStreamSynchronize(st);
-  cudaFree(tmp);
+  if (e2 == cudaSuccess) block_give(B.device, tmp, got);  // the stream is idle
+  else cudaFree(tmp);
   if (s) return s;
   GBX_CUDA(e, "mixed-form bounds");
   GBX_CUDA(e2, "mixed-form bounds");
@@ -934,18 +929,11 @@ static int ensure_mixed_bounds(Basis& B, cudaStream_t st) {
   return GBX_OK;
 }
 
-// The basis's auxiliary streams (kMaxAuxStreams, made on first use; calls use the first
-// B.n_streams of them) with their join events and the fork event.
+// The basis's streams (taken from the pool on first use), with at least B.n_streams auxiliary ones.
 static int ensure_aux_streams(Basis& B) {
-  if (!B.aux.empty()) return GBX_OK;
-  B.aux.assign(kMaxAuxStreams, nullptr);
-  B.join.assign(kMaxAuxStreams, nullptr);
-  for (int j = 0; j < kMaxAuxStreams; ++j) {
-    GBX_CUDA(cudaStreamCreateWithFlags(&B.aux[j], cudaStreamNonBlocking), "create stream");
-    GBX_CUDA(cudaEventCreateWithFlags(&B.join[j], cudaEventDisableTiming), "create event");
-  }
-  GBX_CUDA(cudaEventCreateWithFlags(&B.fork, cudaEventDisableTiming), "create event");
-  return GBX_OK;
+  int s;
+  if (!B.streams && (s = streams_take(B.device, &B.streams))) return s;
+  return B.streams->ensure_aux(B.n_streams);
 }
 
 namespace {
@@ -1078,8 +1066,8 @@ int run_compact(Basis& B, double tau, cudaStream_t st, double skip, double fp32)
   if ((s = ensure_tickets(B, 2LL * nblk, st, &tickets))) return s;
   if (nstreams) {
     if ((s = ensure_aux_streams(B))) return s;
-    GBX_CUDA(cudaEventRecord(B.fork, st), "fork");
-    for (int j = 0; j < nstreams; ++j) GBX_CUDA(cudaStreamWaitEvent(B.aux[j], B.fork, 0), "fork wait");
+    GBX_CUDA(cudaEventRecord(B.streams->fork, st), "fork");
+    for (int j = 0; j < nstreams; ++j) GBX_CUDA(cudaStreamWaitEvent(B.streams->aux[j], B.streams->fork, 0), "fork wait");
   }
   if (zero_list) {
     // on the caller's stream, beside the class blocks (disjoint entries of the store)
@@ -1092,7 +1080,7 @@ int run_compact(Basis& B, double tau, cudaStream_t st, double skip, double fp32)
   }
   for (int i = 0; i < nblk; ++i) {
     const int k = B.launch_order.empty() ? i : B.launch_order[i];
-    const cudaStream_t bs = nstreams ? B.aux[i % nstreams] : st;
+    const cudaStream_t bs = nstreams ? B.streams->aux[i % nstreams] : st;
     const HostBlock& h = B.blocks[k];
     int la, lb, lc, ld;
     class_dims(h.cb, la, lb);
@@ -1127,15 +1115,15 @@ int run_compact(Basis& B, double tau, cudaStream_t st, double skip, double fp32)
       a.ticket = tickets ? tickets + 2 * k + 1 : nullptr;
       const int grid32 = (int)std::max<long long>(
           1, std::min<long long>((n32 * h.team + 127) / 128, (long long)nsm * h.ctas_per_sm));
-      const cudaStream_t bs32 = nstreams ? B.aux[(i + 1) % nstreams] : st;
+      const cudaStream_t bs32 = nstreams ? B.streams->aux[(i + 1) % nstreams] : st;
       if ((s = launch_class(la, lb, lc, ld, a, grid32, bs32))) return s;
     }
   }
   if (per_block) cudaEventRecord(B.blk_ev[nblk], st);
   if (nstreams) {
     for (int j = 0; j < nstreams; ++j) {
-      GBX_CUDA(cudaEventRecord(B.join[j], B.aux[j]), "join");
-      GBX_CUDA(cudaStreamWaitEvent(st, B.join[j], 0), "join wait");
+      GBX_CUDA(cudaEventRecord(B.streams->join[j], B.streams->aux[j]), "join");
+      GBX_CUDA(cudaStreamWaitEvent(st, B.streams->join[j], 0), "join wait");
     }
   }
   return GBX_OK;
@@ -1334,8 +1322,8 @@ int run_coulomb(Basis& B, const double* D, double tau, double* J, cudaStream_t s
     cudaEventRecord(B.blk_ev[nblk], st);
     return GBX_OK;
   }
-  GBX_CUDA(cudaEventRecord(B.fork, st), "fork");
-  for (int j = 0; j < nstreams; ++j) GBX_CUDA(cudaStreamWaitEvent(B.aux[j], B.fork, 0), "fork wait");
+  GBX_CUDA(cudaEventRecord(B.streams->fork, st), "fork");
+  for (int j = 0; j < nstreams; ++j) GBX_CUDA(cudaStreamWaitEvent(B.streams->aux[j], B.streams->fork, 0), "fork wait");
   // largest lists first, round robin over the streams
   std::vector<int> order(lists.size());
   for (size_t i = 0; i < order.size(); ++i) order[i] = (int)i;
@@ -1346,11 +1334,11 @@ int run_coulomb(Basis& B, const double* D, double tau, double* J, cudaStream_t s
   });
   for (size_t oi = 0; oi < order.size(); ++oi) {
     const int j = (int)(oi % nstreams);
-    if ((s = launch_list(order[oi], B.aux[j], B.d_jwork + (size_t)j * chunk))) return s;
+    if ((s = launch_list(order[oi], B.streams->aux[j], B.d_jwork + (size_t)j * chunk))) return s;
   }
   for (int j = 0; j < nstreams; ++j) {
-    GBX_CUDA(cudaEventRecord(B.join[j], B.aux[j]), "join");
-    GBX_CUDA(cudaStreamWaitEvent(st, B.join[j], 0), "join wait");
+    GBX_CUDA(cudaEventRecord(B.streams->join[j], B.streams->aux[j]), "join");
+    GBX_CUDA(cudaStreamWaitEvent(st, B.streams->join[j], 0), "join wait");
   }
   return GBX_OK;
 }
@@ -1455,7 +1443,11 @@ int run_full_host(Basis& B, int notation, double tau, double* out_host, cudaStre
     GBX_CUDA(cudaStreamSynchronize(st), "synchronize");
     return GBX_OK;
   }
-  const long long xs = std::max<long long>(1, (long long)(kStageBytes / (slab * sizeof(double))));
+  // at least kStageSlabs slabs, so that expansion, device-to-host copy and the copy out of the ring
+  // overlap on small tensors too (a 50 MB tensor in one slab: each after the other)
+  const size_t target = std::min(kStageBytes, std::max(kOneThreadCopy, (size_t)n * slab *
+                                                       sizeof(double) / kStageSlabs));
+  const long long xs = std::max<long long>(1, (long long)(target / (slab * sizeof(double))));
   const size_t chunk = (size_t)std::min<long long>(xs, n) * slab;
   if (B.stage_elems < chunk) {
     if (B.d_stage) {
@@ -1468,13 +1460,7 @@ int run_full_host(Basis& B, int notation, double tau, double* out_host, cudaStre
       return s;
     B.stage_elems = chunk;
   }
-  if (!B.copy_stream) {
-    GBX_CUDA(cudaStreamCreateWithFlags(&B.copy_stream, cudaStreamNonBlocking), "create stream");
-    for (int k = 0; k < kStageBuffers; ++k) {
-      GBX_CUDA(cudaEventCreateWithFlags(&B.stage_ready[k], cudaEventDisableTiming), "event");
-      GBX_CUDA(cudaEventCreateWithFlags(&B.stage_free[k], cudaEventDisableTiming), "event");
-    }
-  }
+  if ((s = ensure_aux_streams(B))) return s;
   if ((s = run_compact(B, tau, st))) return s;
   const ExpandArgs e = expand_args(B, notation, nullptr);
   const int nsm = num_sms(B.device);
@@ -1498,7 +1484,7 @@ int run_full_host(Basis& B, int notation, double tau, double* out_host, cudaStre
     const long long x0 = (long long)i * xs, x1 = std::min(n, x0 + xs);
     const int k = i % kStageBuffers;
     double* buf = B.d_stage + (size_t)k * B.stage_elems;
-    if (i >= kStageBuffers) GBX_CUDA(cudaStreamWaitEvent(st, B.stage_free[k], 0), "wait slab");
+    if (i >= kStageBuffers) GBX_CUDA(cudaStreamWaitEvent(st, B.streams->stage_free[k], 0), "wait slab");
     const long long planes = (x1 - x0) * n;
     const int grid = (int)std::max<long long>(1, std::min<long long>(planes, (long long)nsm * per_sm));
     ExpandArgs es = e;  // this launch's destination: the slab
@@ -1506,22 +1492,29 @@ int run_full_host(Basis& B, int notation, double tau, double* out_host, cudaStre
     es.out_len = (x1 - x0) * slab;
     expand_slab<<<grid, 512, row_bytes, st>>>(es, x0, x1, buf);
     GBX_CUDA(cudaGetLastError(), "expand_slab launch");
-    GBX_CUDA(cudaEventRecord(B.stage_ready[k], st), "record slab");
-    GBX_CUDA(cudaStreamWaitEvent(B.copy_stream, B.stage_ready[k], 0), "wait slab");
+    GBX_CUDA(cudaEventRecord(B.streams->stage_ready[k], st), "record slab");
+    GBX_CUDA(cudaStreamWaitEvent(B.streams->copy, B.streams->stage_ready[k], 0), "wait slab");
     double* dst = pinned ? out_host + (size_t)x0 * slab : hring + (size_t)k * chunk;
     GBX_CUDA(cudaMemcpyAsync(dst, buf, (size_t)(x1 - x0) * slab * sizeof(double),
-                             cudaMemcpyDeviceToHost, B.copy_stream),
+                             cudaMemcpyDeviceToHost, B.streams->copy),
              "copy slab to host");
-    GBX_CUDA(cudaEventRecord(B.stage_free[k], B.copy_stream), "record slab copy");
+    GBX_CUDA(cudaEventRecord(B.streams->stage_free[k], B.streams->copy), "record slab copy");
     return GBX_OK;
   };
   if (pinned) {
     for (int i = 0; i < nslab; ++i)
       if ((s = issue(i))) return s;
+  } else if (nslab == 1 && chunk * sizeof(double) <= kOneThreadCopy) {
+    if ((s = issue(0))) return s;
+    GBX_CUDA(cudaEventSynchronize(B.streams->stage_free[0]), "slab copy");
+    std::memcpy(out_host, hring, chunk * sizeof(double));
   } else {
     // workers copy their share of each slab once its device-to-host copy has finished; slab
     // i + kStageBuffers reuses ring slot i % kStageBuffers only after every worker is done
-    const int nthr = (int)std::max(1u, std::min(16u, std::thread::hardware_concurrency() / 2));
+    // a thread for every 4 MB of the tensor: starting one takes as long as copying some 100 KB
+    const size_t bytes = (size_t)n * slab * sizeof(double);
+    const int nthr = (int)std::max<size_t>(
+        1, std::min<size_t>({(size_t)16, std::thread::hardware_concurrency() / 2u, bytes >> 22}));
     std::atomic<int> issued{0}, failed{0};
     std::unique_ptr<std::atomic<int>[]> done(new std::atomic<int>[nslab]);
     for (int i = 0; i < nslab; ++i) done[i].store(0);
@@ -1531,7 +1524,7 @@ int run_full_host(Basis& B, int notation, double tau, double* out_host, cudaStre
           if (failed.load()) return;
           std::this_thread::yield();
         }
-        if (cudaEventSynchronize(B.stage_free[i % kStageBuffers]) != cudaSuccess) {
+        if (cudaEventSynchronize(B.streams->stage_free[i % kStageBuffers]) != cudaSuccess) {
           failed.store(1);
         } else {
           const long long x0 = (long long)i * xs, x1 = std::min(n, x0 + xs);
@@ -1560,7 +1553,7 @@ int run_full_host(Basis& B, int notation, double tau, double* out_host, cudaStre
     if (s) return s;
     if (failed.load()) return set_error(GBX_ERR_CUDA, "slab copy to host failed");
   }
-  GBX_CUDA(cudaStreamSynchronize(B.copy_stream), "synchronize copies");
+  GBX_CUDA(cudaStreamSynchronize(B.streams->copy), "synchronize copies");
   GBX_CUDA(cudaStreamSynchronize(st), "synchronize");
   return GBX_OK;
 }

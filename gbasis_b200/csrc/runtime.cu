@@ -203,48 +203,107 @@ static void cache_give(int device, void* p, size_t bytes) {
   cudaFree(p);
 }
 
+int block_alloc(int device, void** p, size_t bytes, size_t* got, const char* what) {
+  if (bytes == 0) bytes = 16;
+  *p = cache_take(device, bytes, got);
+  if (!*p) {
+    GBX_CUDA(cudaMalloc(p, bytes), what);
+    *got = bytes;
+  }
+  return GBX_OK;
+}
+
+void block_give(int device, void* p, size_t bytes) { cache_give(device, p, bytes); }
+
+// ------------------------------------------------------------------- stream pool
+constexpr int kPooledStreamSets = 4;  // idle sets kept per device
+// under g_block_mu; never destroyed (the driver may be gone when static destructors run)
+static std::vector<std::unique_ptr<StreamSet>>& g_stream_sets =
+    *new std::vector<std::unique_ptr<StreamSet>>;
+
+int StreamSet::ensure_aux(int n) {
+  while ((int)aux.size() < n) {
+    cudaStream_t s = nullptr;
+    cudaEvent_t e = nullptr;
+    GBX_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking), "create stream");
+    aux.push_back(s);
+    GBX_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "create event");
+    join.push_back(e);
+  }
+  return GBX_OK;
+}
+
+StreamSet::~StreamSet() {
+  DeviceGuard g(device);
+  for (cudaStream_t s : aux) cudaStreamDestroy(s);
+  for (cudaEvent_t e : join) cudaEventDestroy(e);
+  for (cudaEvent_t e : {fork, in, out})
+    if (e) cudaEventDestroy(e);
+  if (copy) cudaStreamDestroy(copy);
+  for (cudaEvent_t e : stage_ready)
+    if (e) cudaEventDestroy(e);
+  for (cudaEvent_t e : stage_free)
+    if (e) cudaEventDestroy(e);
+}
+
+int streams_take(int device, std::unique_ptr<StreamSet>* out) {
+  {
+    std::lock_guard<std::mutex> lk(g_block_mu);
+    for (size_t i = 0; i < g_stream_sets.size(); ++i)
+      if (g_stream_sets[i]->device == device) {
+        *out = std::move(g_stream_sets[i]);
+        g_stream_sets.erase(g_stream_sets.begin() + i);
+        return GBX_OK;
+      }
+  }
+  auto set = std::make_unique<StreamSet>();
+  set->device = device;
+  for (cudaEvent_t* e : {&set->fork, &set->in, &set->out})
+    GBX_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming), "create event");
+  GBX_CUDA(cudaStreamCreateWithFlags(&set->copy, cudaStreamNonBlocking), "create stream");
+  for (int k = 0; k < kStageBuffers; ++k) {
+    GBX_CUDA(cudaEventCreateWithFlags(&set->stage_ready[k], cudaEventDisableTiming), "event");
+    GBX_CUDA(cudaEventCreateWithFlags(&set->stage_free[k], cudaEventDisableTiming), "event");
+  }
+  *out = std::move(set);
+  return GBX_OK;
+}
+
+void streams_give(std::unique_ptr<StreamSet> set, bool idle) {
+  if (!set || !idle) return;  // a set that may still have work is destroyed, not shared
+  std::lock_guard<std::mutex> lk(g_block_mu);
+  int held = 0;
+  for (const auto& s : g_stream_sets) held += s->device == set->device;
+  if (held < kPooledStreamSets) g_stream_sets.push_back(std::move(set));
+}
+
 Basis::~Basis() {
   // A basis that never allocated device memory nor created a stream or event (host
   // bookkeeping only, as the allocation-free entry point uses it) touches no device state
   // here: no device switch and no device-wide synchronisation.
-  bool owns = !dev_allocs.empty() || fork || copy_stream || !aux.empty() || !join.empty() ||
-              !blk_ev.empty();
+  bool owns = !dev_allocs.empty() || streams || !blk_ev.empty();
   for (cudaEvent_t e : ev) owns = owns || e;
-  for (cudaEvent_t e : stage_ready) owns = owns || e;
-  for (cudaEvent_t e : stage_free) owns = owns || e;
   if (!owns) return;
   DeviceGuard g(device);
   // blocks go back to the cache only once nothing queued on the device can still use them
   // (what cudaFree would have waited for)
-  if (cudaDeviceSynchronize() == cudaSuccess) {
+  const bool idle = cudaDeviceSynchronize() == cudaSuccess;
+  if (idle) {
     for (auto& a : dev_allocs) cache_give(device, a.first, a.second);
   } else {
     for (auto& a : dev_allocs) cudaFree(a.first);
   }
+  streams_give(std::move(streams), idle);
   for (cudaEvent_t& e : ev)
     if (e) cudaEventDestroy(e);
   for (cudaEvent_t& e : blk_ev)
     if (e) cudaEventDestroy(e);
-  for (cudaStream_t& x : aux)
-    if (x) cudaStreamDestroy(x);
-  for (cudaEvent_t& e : join)
-    if (e) cudaEventDestroy(e);
-  if (fork) cudaEventDestroy(fork);
-  for (cudaEvent_t& e : stage_ready)
-    if (e) cudaEventDestroy(e);
-  for (cudaEvent_t& e : stage_free)
-    if (e) cudaEventDestroy(e);
-  if (copy_stream) cudaStreamDestroy(copy_stream);
 }
 
 int Basis::alloc(void** p, size_t bytes, const char* what) {
-  if (bytes == 0) bytes = 16;
   size_t got = 0;
-  *p = cache_take(device, bytes, &got);
-  if (!*p) {
-    GBX_CUDA(cudaMalloc(p, bytes), what);
-    got = bytes;
-  }
+  const int s = block_alloc(device, p, bytes, &got, what);
+  if (s) return s;
   dev_allocs.push_back({*p, got});
   return GBX_OK;
 }
@@ -531,9 +590,11 @@ int gbx_basis_set_potential(gbx_basis* b, int potential, double omega) {
 
 int gbx_release_cached_memory(void) {
   std::vector<CachedBlock> blocks;
+  std::vector<std::unique_ptr<StreamSet>> sets;  // destroyed at the end, outside the lock
   {
     std::lock_guard<std::mutex> lk(g_block_mu);
     blocks.swap(g_blocks);
+    sets.swap(g_stream_sets);
   }
   for (const CachedBlock& b : blocks) {
     DeviceGuard g(b.device);
@@ -724,6 +785,17 @@ int gbx_block_info(const gbx_basis* b, int k, int* cls4, int* team, double* avg_
   if (team) *team = h.team;
   if (avg_prims) *avg_prims = h.avg_prims;
   if (n_quartets) *n_quartets = B.counts_on_host ? h.j_computed : h.ncand;
+  return GBX_OK;
+}
+
+int gbx_block_table(const gbx_basis* b, int n, int* cls4, int* team, double* avg_prims,
+                    int64_t* n_quartets) {
+  for (int k = 0; k < n; ++k) {
+    const int s = gbx_block_info(b, k, cls4 ? cls4 + 4 * k : nullptr, team ? team + k : nullptr,
+                                 avg_prims ? avg_prims + k : nullptr,
+                                 n_quartets ? n_quartets + k : nullptr);
+    if (s) return s;
+  }
   return GBX_OK;
 }
 

@@ -260,6 +260,10 @@ int gbx_phase_times(gbx_basis* b, double* ms3);
 int gbx_num_blocks(const gbx_basis* b, int* n);
 int gbx_block_info(const gbx_basis* b, int k, int* cls4, int* team, double* avg_prims,
                    int64_t* n_quartets);
+/* gbx_block_info of the first n blocks at once: cls4 (4 n), team (n), avg_prims (n), n_quartets
+ * (n); null arrays are left out. */
+int gbx_block_table(const gbx_basis* b, int n, int* cls4, int* team, double* avg_prims,
+                    int64_t* n_quartets);
 int gbx_set_team(gbx_basis* b, int k, int team);
 /* Further launch knobs of block k: variant 0 runs a heavy class on the quadrature kernel (the
  * default), 1 on the line kernel, a warp per quartet, 2 on the split register kernel where the
