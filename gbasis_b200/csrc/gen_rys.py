@@ -257,8 +257,9 @@ def rys_points(n, T):
 
 def root_table(n):
     """Doubles of the n-point table: per unit interval [i, i + 1) of T the coefficients of the
-    polynomials in u = 2 (T - i) - 1, degree by degree (x, w) of each point; then the Hermite limit
-    (x T, w sqrt(T)) of each point."""
+    polynomials in u = 2 (T - i) - 1, two degrees at a time (x, w of degree 2d, x, w of degree
+    2d + 1: one 32-byte load) for each point; then the Hermite limit (x T, w sqrt(T), 0, 0) of each
+    point."""
     import numpy as np
     ld = np.longdouble
     k = np.arange(DEG + 1)
@@ -278,12 +279,13 @@ def root_table(n):
         coef[:, 0] += dd[:, j]
     big = ld(400)
     hx, hw = rys_points(n, [big])
-    tail = np.stack([hx[0] * big, hw[0] * np.sqrt(big)], -1)
-    return [float(v) for v in np.concatenate([coef.reshape(-1), tail.reshape(-1)])]
+    tail = np.stack([hx[0] * big, hw[0] * np.sqrt(big), 0 * big * hx[0], 0 * big * hx[0]], -1)
+    pairs = coef.reshape(TMAX[n], (DEG + 1) // 2, 2, n, 2).transpose(0, 1, 3, 2, 4)
+    return [float(v) for v in np.concatenate([pairs.reshape(-1), tail.reshape(-1)])]
 
 
 def table_offset(n):
-    return sum((TMAX[m] * (DEG + 1) + 1) * m * 2 for m in TMAX if m < n)
+    return sum((TMAX[m] * (DEG + 1) + 2) * m * 2 for m in TMAX if m < n)
 
 
 # ------------------------------------------------------------------------------ code
@@ -405,12 +407,12 @@ def emit_sources(outdir, classes, nfiles=12):
         _put(os.path.join(outdir, name), "\n".join(out) + "\n")
         files.append(name)
     path = os.path.join(outdir, "rys_tables.cu")
-    head = f"// Generated by gen_rys.py: points and weights, degree {DEG} on unit intervals, ranges {TMAX}."
+    head = f"// Generated by gen_rys.py: points and weights, degree {DEG} on unit intervals, two degrees a row, ranges {TMAX}."
     if not (os.path.exists(path) and open(path).readline().rstrip("\n") == head):
         vals = [v for n in TMAX for v in root_table(n)]
         text = "\n".join([
             head, '#include "../rys_kernel.cuh"', "namespace gbx {",
-            f"__device__ const double kRysTable[{len(vals)}] = {{",
+            f"__device__ __align__(32) const double kRysTable[{len(vals)}] = {{",
             ",\n".join(", ".join(v.hex() for v in vals[i:i + 6]) for i in range(0, len(vals), 6)),
             "};",
             "// Address of the table on the current device (resolved once per device).",

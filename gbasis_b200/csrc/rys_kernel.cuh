@@ -3,23 +3,29 @@
 // [e0|f0] of a primitive quartet is a sum over n = L/2 + 1 Rys points of Ix Iy Iz (plan and
 // tables: gen_rys.py), so the points of all primitive quartets of a contracted quartet form one
 // long contraction index k.  Per chunk of up to kRysKC points:
-//   points: thread k evaluates its point's abscissa and weight (piecewise polynomials of T) and
-//           writes the recursion coefficients P[.][k];
+//   points: a warp per chunk, lane k its point's abscissa and weight (piecewise polynomials of T)
+//           and the recursion coefficients PR[.][k];
 //   tables: threads (axis, k) run the two-index recursion and write I[axis][(e, f)][k];
 //   sums:   the warps run the columns' matrix products X Y * Z over the chunk on the FP64 matrix
-//           instruction, sums in registers (C::gemm).
+//           instruction, sums in registers (C::gemm), beside the next chunk's tables where two
+//           table buffers fit.
 // The tables have k innermost: a matrix operand is 8 table rows x 4 points.  After the last chunk
-// the sums go to shared memory ACC[e][f] once and
-// the whole CTA runs the tail: horizontal recursions, transforms, store / Schwarz maximum /
-// Coulomb contributions.
+// the sums go to shared memory ACC[e][f] once and the whole CTA runs the tail: horizontal
+// recursions, transforms, store / Schwarz maximum / Coulomb contributions.
 //
-// What bounds it: shared-memory bandwidth (80 to 90 % of the LSU data pipe on (pd|sd), (pf|sf),
-// (df|sf), (pd|pd); FP64 pipe 45 to 55 %).  The matrix instruction is there for its operand reuse:
+// What bounds it: shared memory and the matrix pipe together (l1tex data pipe 64 to 69 %, FP64
+// matrix pipe 52 to 54 % on (dd|dd) and (df|sf) of 81 primitive quartets; (pd|sd) 69 and 34 %), with
+// the barriers between the phases.  The matrix instruction is there for its operand reuse:
 // the same sums with a lane per column and FMAs read 8 shared values for every 9 FMAs and took 1.4
 // to 2 times longer.  Measured on the 20-atom chain's first 10 atoms (spherical, unique integrals,
 // blocks one after another), the line or split kernel before against this one: all heavy classes
 // 97.6 -> 17.9 ms; (pf|sf) 5.05 -> 0.89, (df|pf) 5.24 -> 0.50, (ff|ff) 2.03 -> 0.14, (pd|pd) 2.38
-// -> 0.32 ms (12.3 TF/s of algorithmic work, 36 % of the FP64 rate).  Error against 64-bit
+// -> 0.32 ms (12.3 TF/s of algorithmic work, 36 % of the FP64 rate).  The points of kW chunks at a
+// time (their latency once, not per chunk), the second table buffer, 32-byte table loads and the
+// element offsets of the store kept per row and column then took 3,000 to 20,000 quartets per class
+// of 81 primitive quartets from 33,400 to 29,200 SM cycles a quartet on (dd|dd), 30,400 to 27,500
+// on (df|sf), 6,640 to 6,140 on (pd|sd) (all classes: 8 % less; of 16 primitive quartets 6 % less,
+// of one 2 % more).  Error against 64-bit
 // reference values: tensors of the 60-molecule batch 2.0e-13 before, 2.8e-14 now.
 //
 // Mathematics: [e0|f0] as gbasis/integrals/_two_elec_int.py:293-547 defines it (the engine's other
@@ -46,7 +52,7 @@ __host__ __device__ constexpr int rys_tmax(int n) {
 // Doubles before the n-point table.
 __host__ __device__ constexpr int rys_table_offset(int n) {
   int o = 0;
-  for (int m = 3; m < n; ++m) o += (rys_tmax(m) * (kRysDeg + 1) + 1) * m * 2;
+  for (int m = 3; m < n; ++m) o += (rys_tmax(m) * (kRysDeg + 1) + 2) * m * 2;
   return o;
 }
 int rys_table(const double** out);
@@ -55,27 +61,41 @@ __host__ __device__ constexpr int rys_tet(int k) { return k * (k + 1) * (k + 2) 
 // Components of total angular momentum lo..hi.
 __host__ __device__ constexpr int rys_ncomp(int lo, int hi) { return rys_tet(hi + 1) - rys_tet(lo); }
 
-// Abscissa (in t^2) and weight of point r of the N-point rule for exp(-T t^2) on [0, 1].
+// A 32-byte load of a table row (the address a multiple of 32 bytes).
+struct RysRow4 {
+  double x0, w0, x1, w1;
+};
+__device__ __forceinline__ RysRow4 rys_row(const double* p) {
+  RysRow4 r;
+  asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
+      : "=d"(r.x0), "=d"(r.w0), "=d"(r.x1), "=d"(r.w1)
+      : "l"(p));
+  return r;
+}
+
+// Abscissa (in t^2) and weight of point r of the N-point rule for exp(-T t^2) on [0, 1].  A chunk's
+// lanes gather from as many intervals as it has primitive quartets, so the loads cost wavefronts by
+// count: two degrees of a point's pair of polynomials come in one 32-byte load.
 template <int N>
 __device__ __forceinline__ double2 rys_point(double T, int r, const double* __restrict__ tab) {
-  constexpr int TM = rys_tmax(N);
+  constexpr int TM = rys_tmax(N), ND = (kRysDeg + 1) / 2;
   if (T < (double)TM) {
     const int i = (int)T;
     const double u = fma(2.0, T - (double)i, -1.0);
-    const double2* __restrict__ c =
-        reinterpret_cast<const double2*>(tab) + (size_t)i * (kRysDeg + 1) * N + r;
-    double2 v = __ldg(c + kRysDeg * N);
+    const double* __restrict__ c = tab + ((size_t)i * ND * N + r) * 4;
+    RysRow4 g = rys_row(c + (ND - 1) * N * 4);
+    double x = fma(g.x1, u, g.x0), w = fma(g.w1, u, g.w0);
 #pragma unroll
-    for (int d = kRysDeg - 1; d >= 0; --d) {
-      const double2 g = __ldg(c + d * N);
-      v.x = fma(v.x, u, g.x);
-      v.y = fma(v.y, u, g.y);
+    for (int d = ND - 2; d >= 0; --d) {
+      g = rys_row(c + d * N * 4);
+      x = fma(fma(x, u, g.x1), u, g.x0);
+      w = fma(fma(w, u, g.w1), u, g.w0);
     }
-    return v;
+    return make_double2(x, w);
   }
-  const double2 h = __ldg(reinterpret_cast<const double2*>(tab) + (size_t)TM * (kRysDeg + 1) * N + r);
+  const RysRow4 h = rys_row(tab + ((size_t)TM * ND * N + r) * 4);
   const double q = rsqrt(T);
-  return make_double2(h.x * (q * q), h.y * q);
+  return make_double2(h.x0 * (q * q), h.w0 * q);
 }
 
 // Rows of the per-point coefficients.
@@ -152,9 +172,16 @@ struct RysDims {
   // columns; then the tables and coefficients, overlaid by [e0|cd]
   static constexpr int kAccSize = NE * NFs > 3 * NAB ? NE * NFs : 3 * NAB;
   static constexpr int kAccEven = (kAccSize + 1) & ~1;
-  static constexpr int kTabSize = 3 * TS + kRysRows * kRysKS;
   static constexpr int kHf = C::LD == 0 ? 0 : NE * HS;
-  static constexpr int kSmem = kAccEven + (kTabSize > kHf ? kTabSize : kHf);
+  static constexpr int smem_of(int buffers) {
+    const int t = buffers * 3 * TS + C::kW * kRysRows * kRysKS;
+    return kAccEven + (t > kHf ? t : kHf);
+  }
+  // two table buffers where the CTAs that the registers allow still fit (228 KB per SM; 1 KB and
+  // the shell data of each CTA beside it)
+  static constexpr int kBuf =
+      (long long)kMinCtas * (smem_of(2) * 8 + 16 * (NAB + NKET) + 2 * 1024) <= 228 * 1024 && C::kW > 1 ? 2 : 1;
+  static constexpr int kSmem = smem_of(kBuf);
   // [e0|cd] of classes whose ket pair has no second angular momentum is ACC itself: the bra
   // step's block then sits in the tables' place
   static constexpr int kBlkSize = C::LD == 0 ? kSmem - kAccEven : kAccSize;
@@ -229,18 +256,67 @@ __device__ __forceinline__ void rys_sync() {
   else __syncthreads();
 }
 
+// Points of primitive quartets p0, p0 + 1, ... of a quartet with nk ket primitive pairs (kc points,
+// kpp per primitive quartet): lane k writes its point's recursion coefficients PR[.][k], zeros up to a
+// multiple of 4 points.
+template <int N>
+__device__ __forceinline__ void rys_points(const EriLaunch& a, const PrimPair* __restrict__ bprim,
+                                           const PrimPair* __restrict__ kprim, int nk,
+                                           const double* __restrict__ tab, int p0, int kc, int kpp,
+                                           int lane, double* __restrict__ PR) {
+  if (lane >= ((kc + 3) & ~3)) return;
+  double* const pr = PR + lane;
+  if (lane >= kc) {
+#pragma unroll
+    for (int i = 0; i < kRysRows; ++i) pr[i * kRysKS] = 0.0;
+    return;
+  }
+  const int pi = kpp == N ? lane / N : lane / (2 * N), r2 = lane - pi * kpp, r = r2 < N ? r2 : r2 - N;
+  const int ip = (p0 + pi) / nk, jq = p0 + pi - ip * nk;
+  const PrimPair bp = bprim[ip], kp = kprim[jq];
+  const double rs = rsqrt(bp.zeta + kp.zeta), inv = rs * rs;
+  const double PQx = bp.Px - kp.Px, PQy = bp.Py - kp.Py, PQz = bp.Pz - kp.Pz;
+  const double rz = kp.zeta * inv, re = bp.zeta * inv;  // rho / zeta, rho / eta
+  const double rho = bp.zeta * rz;
+  double T = fmax(rho * fma(PQx, PQx, fma(PQy, PQy, PQz * PQz)), 0.0);
+  double pref = bp.C * kp.C * rs, sx = 1.0;
+  if (a.potential == 1 || r2 >= N) {
+    // erf(omega r)/r: points and weights at s T, scaled by s and sqrt(s); erfc: subtracted
+    const double w2 = a.omega * a.omega;
+    sx = w2 / (w2 + rho);
+    T *= sx;
+    pref *= a.potential == 1 ? sqrt(sx) : -sqrt(sx);
+  }
+  const double2 xw = rys_point<N>(T, r, tab);
+  const double x = xw.x * sx;
+  const double o2z = 0.5 * bp.izeta, o2e = 0.5 * kp.izeta, xz = x * rz, xe = x * re;
+  pr[kB00 * kRysKS] = 0.5 * x * inv;
+  pr[kB10 * kRysKS] = fma(-xz, o2z, o2z);
+  pr[kB01 * kRysKS] = fma(-xe, o2e, o2e);
+  pr[kC0 * kRysKS] = fma(-xz, PQx, bp.Xx);
+  pr[(kC0 + 1) * kRysKS] = fma(-xz, PQy, bp.Xy);
+  pr[(kC0 + 2) * kRysKS] = fma(-xz, PQz, bp.Xz);
+  pr[kD0 * kRysKS] = fma(xe, PQx, kp.Xx);
+  pr[(kD0 + 1) * kRysKS] = fma(xe, PQy, kp.Xy);
+  pr[(kD0 + 2) * kRysKS] = fma(xe, PQz, kp.Xz);
+  pr[kWt * kRysKS] = pref * xw.y;
+}
+
 template <class C>
 __global__ void __launch_bounds__(32 * C::kW, RysDims<C>::kMinCtas) eri_rys(const RysArgs A) {
   using D = RysDims<C>;
-  constexpr int N = C::kN, NT = D::NT, LA = C::LA, LB = C::LB, LC = C::LC, LD = C::LD;
+  constexpr int N = C::kN, NT = D::NT, NW = C::kW, LA = C::LA, LB = C::LB, LC = C::LC, LD = C::LD;
   extern __shared__ __align__(16) double smem[];
   __shared__ RysShells S;
   __shared__ long long s_next[2];
+  // mode 0: element offsets and scales of the block's rows (a, b) and columns (c, d)
+  __shared__ long long s_ro[D::NAB], s_co[D::NKET];
+  __shared__ double s_rs[D::NAB], s_cs[D::NKET];
   const EriLaunch& a = A.a;
   const int tid = threadIdx.x, lane = tid & 31, wq = tid >> 5;
   double* const ACC = smem;
   double* const T = smem + D::kAccEven;
-  double* const PR = T + 3 * D::TS;
+  double* const PR = T + D::kBuf * 3 * D::TS;
   double* const HF = LD == 0 ? ACC : T;
   double* const BLK = LD == 0 ? T : ACC;
   const double* __restrict__ tab = A.tab + rys_table_offset(N);
@@ -253,7 +329,7 @@ __global__ void __launch_bounds__(32 * C::kW, RysDims<C>::kMinCtas) eri_rys(cons
   int turn = 0;
   if (a.ticket) {  // quartets from the launch's counter; the next draw overlaps the quartet
     if (tid == 0) s_next[0] = (long long)atomicAdd(a.ticket, 1ull);
-    rys_sync<C::kW>();
+    rys_sync<NW>();
     w = s_next[0];
   }
   while (w < count) {  // w is the same for all threads of the CTA
@@ -280,66 +356,46 @@ __global__ void __launch_bounds__(32 * C::kW, RysDims<C>::kMinCtas) eri_rys(cons
     for (int i = 0; i < C::kAcc; ++i) acc[i] = 0.0;
     // points per primitive quartet: erfc(omega r)/r is 1/r minus erf(omega r)/r
     const int kpp = a.potential == 2 ? 2 * N : N;
-    const int per_chunk = kRysKC / kpp;
-    for (int p0 = 0; p0 < np; p0 += per_chunk) {
-      const int kc = min(per_chunk, np - p0) * kpp, kcp = (kc + 3) & ~3;
-      // ---- points: by the last warp, whose share of the sums is the lightest
-      if (wq == C::kW - 1 && lane < kcp) {
-        const int k = lane;
-        double* const pr = PR + k;
-        if (k < kc) {
-          const int pi = k / kpp, r2 = k - pi * kpp, r = r2 < N ? r2 : r2 - N;
-          const int ip = (p0 + pi) / nkp, jq = p0 + pi - ip * nkp;
-          const PrimPair bp = bprim[ip], kp = kprim[jq];
-          const double rs = rsqrt(bp.zeta + kp.zeta), inv = rs * rs;
-          const double PQx = bp.Px - kp.Px, PQy = bp.Py - kp.Py, PQz = bp.Pz - kp.Pz;
-          const double rz = kp.zeta * inv, re = bp.zeta * inv;  // rho / zeta, rho / eta
-          const double rho = bp.zeta * rz;
-          double Tq = fmax(rho * fma(PQx, PQx, fma(PQy, PQy, PQz * PQz)), 0.0);
-          double pref = bp.C * kp.C * rs, sx = 1.0;
-          if (a.potential) {
-            // erf(omega r)/r: points and weights at s T, scaled by s and sqrt(s)
-            const bool att = a.potential == 1 || r2 >= N;
-            const double w2 = a.omega * a.omega;
-            if (att) {
-              sx = w2 / (w2 + rho);
-              Tq *= sx;
-              pref *= a.potential == 1 ? sqrt(sx) : -sqrt(sx);
-            }
-          }
-          const double2 xw = rys_point<N>(Tq, r, tab);
-          const double x = xw.x * sx;
-          const double o2z = 0.5 * bp.izeta, o2e = 0.5 * kp.izeta, xz = x * rz, xe = x * re;
-          pr[kB00 * kRysKS] = 0.5 * x * inv;
-          pr[kB10 * kRysKS] = fma(-xz, o2z, o2z);
-          pr[kB01 * kRysKS] = fma(-xe, o2e, o2e);
-          pr[kC0 * kRysKS] = fma(-xz, PQx, bp.Xx);
-          pr[(kC0 + 1) * kRysKS] = fma(-xz, PQy, bp.Xy);
-          pr[(kC0 + 2) * kRysKS] = fma(-xz, PQz, bp.Xz);
-          pr[kD0 * kRysKS] = fma(xe, PQx, kp.Xx);
-          pr[(kD0 + 1) * kRysKS] = fma(xe, PQy, kp.Xy);
-          pr[(kD0 + 2) * kRysKS] = fma(xe, PQz, kp.Xz);
-          pr[kWt * kRysKS] = pref * xw.y;
-        } else {
-#pragma unroll
-          for (int i = 0; i < kRysRows; ++i) pr[i * kRysKS] = 0.0;
-        }
-      }
-      rys_sync<C::kW>();  // points written; the previous chunk's tables are read
-      // ---- tables
+    const int per_chunk = a.potential == 2 ? kRysKC / (2 * N) : kRysKC / N;
+    // tables of chunk c (points PR[c]) into buffer b
+    auto tables = [&](int c, int kcp, int b) {
       for (int i = tid; i < 3 * kcp; i += NT) {
         const int ax = i / kcp, k = i - ax * kcp;
-        const double* const pr = PR + k;
-        rys_axis<D::NE1, D::NF1, D::RF>(pr[(kC0 + ax) * kRysKS], pr[(kD0 + ax) * kRysKS], pr[kB00 * kRysKS],
-                                 pr[kB10 * kRysKS], pr[kB01 * kRysKS],
-                                 ax == 2 ? pr[kWt * kRysKS] : 1.0, T + ax * D::TS + k);
+        const double* const pr = PR + c * kRysRows * kRysKS + k;
+        rys_axis<D::NE1, D::NF1, D::RF>(pr[(kC0 + ax) * kRysKS], pr[(kD0 + ax) * kRysKS],
+                                        pr[kB00 * kRysKS], pr[kB10 * kRysKS], pr[kB01 * kRysKS],
+                                        ax == 2 ? pr[kWt * kRysKS] : 1.0,
+                                        T + (b * 3 + ax) * D::TS + k);
       }
-      rys_sync<C::kW>();
-      // ---- sums
-      C::gemm(wq, lane, T, kcp, acc);
+    };
+    for (int s0 = 0; s0 < np; s0 += NW * per_chunk) {
+      // a chunk per warp, the last warp first (its share of the sums is the lightest): the points'
+      // latency (pair data, then table rows at T) is paid once per NW chunks
+      const int mine = NW - 1 - wq, p0 = s0 + mine * per_chunk;
+      rys_points<N>(a, bprim, kprim, nkp, tab, p0, min(max(np - p0, 0), per_chunk) * kpp, kpp, lane,
+                    PR + mine * kRysRows * kRysKS);
+      const int nc = min(NW, (np - s0 + per_chunk - 1) / per_chunk);
+      auto padded = [&](int c) {
+        return (min(np - s0 - c * per_chunk, per_chunk) * kpp + 3) & ~3;
+      };
+      rys_sync<NW>();  // points written; the previous chunk's tables are read
+      if constexpr (D::kBuf == 2) {  // a chunk's tables beside the sums of the one before
+        for (int c = 0; c <= nc; ++c) {
+          if (c < nc) tables(c, padded(c), c & 1);
+          if (c > 0) C::gemm(wq, lane, T + ((c - 1) & 1) * 3 * D::TS, padded(c - 1), acc);
+          if (c < nc) rys_sync<NW>();
+        }
+      } else {
+        for (int c = 0; c < nc; ++c) {
+          if (c > 0) rys_sync<NW>();
+          tables(c, padded(c), 0);
+          rys_sync<NW>();
+          C::gemm(wq, lane, T, padded(c), acc);
+        }
+      }
     }
     C::store(wq, lane, acc, ACC);
-    rys_sync<C::kW>();  // ACC complete, tables read
+    rys_sync<NW>();  // ACC complete, tables read
     // ------------------------------------------------------------------------------ tail
     const int nA = S.nint[0], nB = S.nint[1], nC = S.nint[2], nD = S.nint[3];
     const int ncol = nC * nD;
@@ -355,6 +411,23 @@ __global__ void __launch_bounds__(32 * C::kW, RysDims<C>::kMinCtas) eri_rys(cons
                  S.scl[1][ub];
         VAB[i] = 0.0;
       }
+    }
+    if (a.mode == 0) {  // read after the barriers below
+      long long bbase, bcols;
+      block_dest(a, P, bbase, bcols);
+      const bool tr = quartet_transposed(P, Q);
+      const long long sbra = tr ? 1 : bcols, sket = tr ? bcols : 1;
+      for (int i = tid; i < nA * nB; i += NT) {
+        const int ua = i / nB, ub = i - ua * nB;
+        s_ro[i] = bbase + ((long long)P.fo + S.pos[0][ua] * S.nout[1] + S.pos[1][ub]) * sbra;
+        s_rs[i] = S.scl[0][ua] * S.scl[1][ub];
+      }
+      for (int i = NT - 1 - tid; i < ncol; i += NT) {
+        const int uc = i / nD, ud = i - uc * nD;
+        s_co[i] = ((long long)Q.fo + S.pos[2][uc] * S.nout[3] + S.pos[3][ud]) * sket;
+        s_cs[i] = S.scl[2][uc] * S.scl[3][ud];
+      }
+      if constexpr (LD == 0) rys_sync<NW>();  // the ket step's barrier otherwise
     }
     // ket recursion and transform on D: tasks (row e, component c) -> HF[e][c][ud]
     if constexpr (LD > 0) {
@@ -375,7 +448,7 @@ __global__ void __launch_bounds__(32 * C::kW, RysDims<C>::kMinCtas) eri_rys(cons
 #pragma unroll
         for (int i = 0; i < D::NCD; ++i) HF[e * D::HS + c * D::NCD + i] = o[i];
       }
-      rys_sync<C::kW>();
+      rys_sync<NW>();
     }
     // transform on C, in place: tasks (row e, ud)
     if constexpr (LC >= 2) {
@@ -390,28 +463,20 @@ __global__ void __launch_bounds__(32 * C::kW, RysDims<C>::kMinCtas) eri_rys(cons
 #pragma unroll
           for (int c = 0; c < 2 * LC + 1; ++c) row[c * nD] = y[c];
         }
-        rys_sync<C::kW>();
+        rys_sync<NW>();
       }
     }
     // bra recursion, transforms and output, a block of columns at a time
     const double ABx = P.ABx, ABy = P.ABy, ABz = P.ABz;
     const bool sphA = LA >= 2 && nA != D::NCA;
     const bool block = sphA || coulomb;  // the columns' values meet in BLK[(a, ub)][column]
-    long long bbase, bcols;
-    block_dest(a, P, bbase, bcols);
-    const bool tr = quartet_transposed(P, Q);
-    const long long sbra = tr ? 1 : bcols, sket = tr ? bcols : 1;
     const int rowlen = D::NCA * nB;
     const int cap = block ? D::kBlkSize / rowlen : ncol;
     const int cmax = block ? min(ncol, (cap & 1) ? cap : cap - 1) : ncol;  // odd row stride
     const int CS = cmax | 1;
     double mx = 0.0;
-    auto put = [&](int ua, int ub, int col, double v) {
-      const int uc = col / nD, ud = col - uc * nD;
-      const long long at = bbase +
-                           ((long long)P.fo + S.pos[0][ua] * S.nout[1] + S.pos[1][ub]) * sbra +
-                           ((long long)Q.fo + S.pos[2][uc] * S.nout[3] + S.pos[3][ud]) * sket;
-      out_store(a, at, v * (S.scl[0][ua] * S.scl[1][ub]) * (S.scl[2][uc] * S.scl[3][ud]));
+    auto put = [&](int row, int col, double v) {
+      out_store(a, s_ro[row] + s_co[col], v * s_rs[row] * s_cs[col]);
     };
     for (int c0 = 0; c0 < ncol; c0 += cmax) {
       const int cc = min(cmax, ncol - c0);
@@ -438,11 +503,11 @@ __global__ void __launch_bounds__(32 * C::kW, RysDims<C>::kMinCtas) eri_rys(cons
         for (int i = 0; i < D::NCB; ++i) {
           if (i >= nB) break;
           if (block) BLK[(ca * nB + i) * CS + cl] = o[i];
-          else put(ca, i, col, o[i]);
+          else put(ca * nB + i, col, o[i]);
         }
       }
       if (!block) continue;
-      rys_sync<C::kW>();
+      rys_sync<NW>();
       if constexpr (LA >= 2) {
         if (sphA) {  // transform on A: tasks (ub, column), stored or put back in place
           for (int t = tid; t < cc * nB; t += NT) {
@@ -454,10 +519,10 @@ __global__ void __launch_bounds__(32 * C::kW, RysDims<C>::kMinCtas) eri_rys(cons
 #pragma unroll
             for (int i = 0; i < 2 * LA + 1; ++i) {
               if (coulomb) BLK[(i * nB + ub) * CS + cl] = y[i];
-              else put(i, ub, c0 + cl, y[i]);
+              else put(i * nB + ub, c0 + cl, y[i]);
             }
           }
-          rys_sync<C::kW>();
+          rys_sync<NW>();
         }
       }
       if (coulomb) {
@@ -478,14 +543,14 @@ __global__ void __launch_bounds__(32 * C::kW, RysDims<C>::kMinCtas) eri_rys(cons
             if (Q.shA != Q.shB) j_add(a, fd * a.nbf + fc, s);
           }
         }
-        rys_sync<C::kW>();
+        rys_sync<NW>();
       }
     }
     if (schwarz) {
       for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-      rys_sync<C::kW>();  // HF is read
+      rys_sync<NW>();  // HF is read
       if (lane == 0) smem[wq] = mx;
-      rys_sync<C::kW>();
+      rys_sync<NW>();
       if (tid == 0) {
         for (int i = 1; i < C::kW; ++i) mx = fmax(mx, smem[i]);
         a.qout[pq.x] = sqrt(mx);
@@ -501,7 +566,7 @@ __global__ void __launch_bounds__(32 * C::kW, RysDims<C>::kMinCtas) eri_rys(cons
         if (P.shA != P.shB) j_add(a, fb * a.nbf + fa, s);
       }
     }
-    rys_sync<C::kW>();  // shared memory free for the next quartet; the next draw is visible
+    rys_sync<NW>();  // shared memory free for the next quartet; the next draw is visible
     turn ^= 1;
     w = a.ticket ? s_next[turn] : w + gridDim.x;
   }
@@ -518,7 +583,7 @@ int launch_rys_t(const EriLaunch& a, cudaStream_t st) {
   cudaGetDevice(&dev);
   const int cm = a.mode == 2 ? 1 : 0;
   const int smem = (D::kSmem + (cm ? D::NKET + 2 * D::NAB : 0)) * (int)sizeof(double);
-  static_assert((D::kSmem + D::NKET + 2 * D::NAB) * 8 + 2048 <= kRysMaxSmem, "shared memory");
+  static_assert((D::kSmem + 3 * D::NKET + 4 * D::NAB) * 8 + 1024 <= kRysMaxSmem, "shared memory");
   // CTAs the device keeps resident in this mode, found once per device and mode
   static std::atomic<int> resident[64][2];
   int r = dev >= 0 && dev < 64 ? resident[dev][cm].load() : 0;

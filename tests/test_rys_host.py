@@ -40,12 +40,12 @@ def _points(n, T, tab):
         i = int(T)
         u = 2.0 * (T - i) - 1.0
         c = tab[i * (gen_rys.DEG + 1) * n * 2:(i + 1) * (gen_rys.DEG + 1) * n * 2]
-        c = c.reshape(gen_rys.DEG + 1, n, 2)
+        c = c.reshape(-1, n, 2, 2).transpose(0, 2, 1, 3).reshape(gen_rys.DEG + 1, n, 2)
         v = c[-1].copy()
         for d in range(gen_rys.DEG - 1, -1, -1):
             v = v * u + c[d]
         return v[:, 0], v[:, 1]
-    h = tab[-2 * n:].reshape(n, 2)
+    h = tab[-4 * n:].reshape(n, 4)
     return h[:, 0] / T, h[:, 1] / math.sqrt(T)
 
 
