@@ -2,9 +2,21 @@
 //
 // One thread owns one contracted shell quartet (bra pair p, ket pair q) of a class block:
 // it loops over the primitive quartets, evaluates F_m(T) from a shared-memory Taylor table,
-// runs the generated VRR+ETR into register accumulators [e0|f0], then the generated HRR,
-// the Cartesian->spherical transform (constant code) and the per-function permutation /
+// runs the generated vertical recursion of both sides into register accumulators [e0|f0], then the
+// generated HRR, the Cartesian->spherical transform (constant code) and the per-function permutation /
 // scale, and stores the block into the compact store.
+//
+// Bound: FP64 issue and latency of the recursion, and registers (acc is NE x NF).  So the kernel
+// takes the recursion with the fewest operations and accumulators.  f is raised by its own vertical
+// recursion, not transferred from [e+f|0] (no [e|0] beyond the bra's range: 309 against 420
+// operations on (ds|ds)), and a pair of an s shell and another runs on the other shell (`flip`), so
+// that (sd| is [d0| alone: 36 accumulators and 309 operations on (sd|sd) against 100 and 489, and no
+// horizontal recursion.  Measured, one B200, blocks one after another, before -> now: (sd|sd) of
+// 62,000 quartets of 128 primitive quartets 1.32 -> 0.49 ms, (sd|sp) 1.41 -> 1.01, (sd|pp) 1.42 ->
+// 0.89, (pd|sp) 1.40 -> 1.16; all register classes of the 9-atom direct J 19.3 -> 15.5 ms, of the
+// 60-molecule batch 4.17 -> 3.38, of the 8-atom full tensor 1.54 -> 1.36.  The centre may be far from
+// P without loss: no term of the recursion is multiplied by zeta/eta (tensors of the batch, error
+// against 64-bit reference values: 2.8e-14 before, 1.7e-14 now).
 //
 // Reference mathematics: gbasis/integrals/_two_elec_int.py:293-812 (prefactor, VRR, ETR,
 // contraction, HRR, component norm) and gbasis/base_four_symm.py:195-349 (norm_cont,
@@ -235,19 +247,19 @@ __device__ __forceinline__ void coulomb_epilogue(const EriLaunch& a, int2 pq, co
 }
 
 // R = double: the FP64 form.  R = float: the mixed form's FP32 path — Boys values and the
-// geometric factors are formed in FP64 and rounded, the vertical and transfer recursions run
+// geometric factors are formed in FP64 and rounded, the vertical recursions run
 // in FP32 and [e0|f0] accumulates in FP32 over the lane's primitive quartets; the team
 // reduction, horizontal recursion, transforms and stores are FP64.
 // Resident CTAs per SM a class's register kernel is compiled for.  Classes whose unconstrained
 // register use is 171-200 per thread would fit 2 CTAs of 128 threads per SM; for these the cap
 // of 168 registers that a third CTA needs costs at most a few spilled values, and the extra warps
-// hide more of the primitive-loop latency (measured per class on medium8 and chain20: 8-13 %
-// shorter blocks; classes further above the cap spill heavily and lose).
+// hide more of the primitive-loop latency ((pp|ps) of the 8-atom full tensor 0.090 -> 0.081 ms, of the
+// 60-molecule batch 0.219 -> 0.180; classes further above the cap spill heavily and lose).
 // (ss|ss) keeps the 64 registers that let 8 CTAs (the shared-memory limit) share an SM.
 __host__ __device__ constexpr int eri_min_blocks(int la, int lb, int lc, int ld) {
   return (la + lb + lc + ld == 0) ? 8
-         : ((la == 0 && lb == 2 && lc == 0 && ld == 1) ||
-            (la == 1 && lb == 1 && lc == 0 && ld == 1) || (la == 1 && lb == 3 && lc == 0 && ld == 0))
+         : ((la == 1 && lb == 1 && lc == 1 && ld == 0) ||
+            (la == 2 && lb == 2 && lc == 0 && ld == 0) || (la == 1 && lb == 3 && lc == 0 && ld == 0))
              ? 3
              : 1;
 }
@@ -292,6 +304,8 @@ __global__ void __launch_bounds__(kEriThreads, eri_min_blocks(LA, LB, LC, LD))
 #pragma unroll
     for (int i = 0; i < C::NE * C::NF; ++i) accr[i] = R(0);
 
+    // a flipped pair's recursion centre is its second shell: P - B = (P - A) + (A - B)
+    const bool fb = LB == 0 && LA > 0 && (a.flip & 1), fk = LD == 0 && LC > 0 && (a.flip & 2);
     const int nprim = valid ? P.nprim * Q.nprim : 0;
     int ip = tl / Q.nprim, jq = tl - ip * Q.nprim;
     // one primitive quartet (bra primitive pair ipx, ket jqx) into accr
@@ -311,21 +325,26 @@ __global__ void __launch_bounds__(kEriThreads, eri_min_blocks(LA, LB, LC, LD))
       const double pref = bp.C * kp.C * r;
 #pragma unroll
       for (int m = 0; m <= L; ++m) F[m] *= pref;
-      const double ze = bp.zeta * kp.izeta;
-      const double o2e = 0.5 * kp.izeta;
+      const double o2e = 0.5 * kp.izeta, re = bp.zeta * inv, o2s = 0.5 * inv;  // re = rho / eta
+      double Ax = bp.Xx, Ay = bp.Xy, Az = bp.Xz, Cx = kp.Xx, Cy = kp.Xy, Cz = kp.Xz;
+      if constexpr (LB == 0 && LA > 0) {
+        if (fb) { Ax += P.ABx; Ay += P.ABy; Az += P.ABz; }
+      }
+      if constexpr (LD == 0 && LC > 0) {
+        if (fk) { Cx += Q.ABx; Cy += Q.ABy; Cz += Q.ABz; }
+      }
       if constexpr (sizeof(R) == sizeof(double)) {
-        C::template prim<double>(F, bp.Xx, bp.Xy, bp.Xz, -rz * PQx, -rz * PQy, -rz * PQz, o2z,
-                                 rz, fma(ze, bp.Xx, kp.Xx), fma(ze, bp.Xy, kp.Xy),
-                                 fma(ze, bp.Xz, kp.Xz), ze, o2e, accr);
+        C::template prim<double>(F, Ax, Ay, Az, -rz * PQx, -rz * PQy, -rz * PQz, o2z, rz, Cx, Cy, Cz,
+                                 re * PQx, re * PQy, re * PQz, o2e, re, o2s, accr);
       } else {
         float F32[L + 1];
 #pragma unroll
         for (int m = 0; m <= L; ++m) F32[m] = (float)F[m];
-        C::template prim<float>(F32, (float)bp.Xx, (float)bp.Xy, (float)bp.Xz,
-                                (float)(-rz * PQx), (float)(-rz * PQy), (float)(-rz * PQz),
-                                (float)o2z, (float)rz, (float)fma(ze, bp.Xx, kp.Xx),
-                                (float)fma(ze, bp.Xy, kp.Xy), (float)fma(ze, bp.Xz, kp.Xz),
-                                (float)ze, (float)o2e, accr);
+        C::template prim<float>(F32, (float)Ax, (float)Ay, (float)Az, (float)(-rz * PQx),
+                                (float)(-rz * PQy), (float)(-rz * PQz), (float)o2z, (float)rz,
+                                (float)Cx, (float)Cy, (float)Cz, (float)(re * PQx),
+                                (float)(re * PQy), (float)(re * PQz), (float)o2e, (float)re,
+                                (float)o2s, accr);
       }
     };
     auto advance = [&]() {
@@ -369,10 +388,10 @@ __global__ void __launch_bounds__(kEriThreads, eri_min_blocks(LA, LB, LC, LD))
       continue;
     }
 
-    const ShellDev& sA = a.shells[P.shA];
-    const ShellDev& sB = a.shells[P.shB];
-    const ShellDev& sC = a.shells[Q.shA];
-    const ShellDev& sD = a.shells[Q.shB];
+    const ShellDev& sA = a.shells[fb ? P.shB : P.shA];
+    const ShellDev& sB = a.shells[fb ? P.shA : P.shB];
+    const ShellDev& sC = a.shells[fk ? Q.shB : Q.shA];
+    const ShellDev& sD = a.shells[fk ? Q.shA : Q.shB];
     if (LD >= 2 && sD.sph) sph_axis<LD, NCA * NCB * NCC, 1>(out);
     if (LC >= 2 && sC.sph) sph_axis<LC, NCA * NCB, NCD>(out);
     if (LB >= 2 && sB.sph) sph_axis<LB, NCA, NCC * NCD>(out);

@@ -23,8 +23,8 @@ constexpr int kBoysOrders = kBoysMMax + kBoysTaylor;  // orders stored in the gl
 
 __host__ __device__ constexpr int ncart(int l) { return (l + 1) * (l + 2) / 2; }
 
-// Pair classes are ordered pair types (lA, lB), A being the shell the vertical recursion runs
-// on (the one with the larger exponent, for numerical stability), sorted by
+// Pair classes are ordered pair types (lA, lB), A being the shell with the larger exponent (the
+// one the recursions run on, for numerical stability, but see EriLaunch::flip), sorted by
 // (lA + lB, max(lA, lB), lA).  A quartet's bra is the pair with the larger class index.
 constexpr int kNumPairClasses = (kLMax + 1) * (kLMax + 1);
 constexpr int kPairClassL[kNumPairClasses][2] = {
@@ -137,6 +137,9 @@ struct EriLaunch {
   // heavy classes: 0 = quadrature kernel, 1 = line kernel, 2 = split register kernel (classes that
   // have one) or the line kernel's group form
   int variant;
+  // register and quadrature kernels, set by launch_class: bit 0 the bra pair, bit 1 the ket pair
+  // runs with its second shell as the recursion centre (its first is an s shell)
+  int flip;
   // work counter of this launch, zero before it starts: in the heavy-class kernels warps (split
   // kernel: CTAs) take their next quartets from it with atomicAdd, so that a CTA that becomes
   // resident late (class blocks share the GPU with other blocks on other streams) takes less

@@ -71,7 +71,7 @@ __global__ void __launch_bounds__(128) point_charge_block(const PointArgs a) {
 #pragma unroll
       for (int m = 0; m <= L; ++m) F[m] *= pref;
       C::template prim<double>(F, bp.Xx, bp.Xy, bp.Xz, -PCx, -PCy, -PCz, 0.5 * bp.izeta, 1.0,
-                               0.0, 0.0, 0.0, 0.0, 0.0, acc);
+                               0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, acc);
     }
     double o[C::NAB * C::NCD];
     C::hrr(acc, P.ABx, P.ABy, P.ABz, 0.0, 0.0, 0.0, o);

@@ -392,8 +392,10 @@ int build_basis(Basis& B, int n, const int* angmom, const int* nprim, const doub
   B.h_coefs.assign(coefs, coefs + prim_total);
 
   // pairs: i <= j, stored with the shell of larger maximum exponent first (the vertical
-  // recursion runs on it: P - A stays small, which keeps the Obara-Saika and transfer
-  // recursions from cancelling digits on diffuse partners); ties: higher l, lower index.
+  // recursion runs on it: P - A stays small, which keeps the transfer and horizontal
+  // recursions from cancelling digits on diffuse partners; the register and quadrature kernels,
+  // which transfer nothing, swap a pair whose first shell is an s shell, see EriLaunch::flip);
+  // ties: higher l, lower index.
   // Sorted by (class, nprim desc).
   struct HP {
     int a, b, cls, nprim, i, j;

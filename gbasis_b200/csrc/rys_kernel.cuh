@@ -29,7 +29,7 @@
 // reference values: tensors of the 60-molecule batch 2.0e-13 before, 2.8e-14 now.
 //
 // Mathematics: [e0|f0] as gbasis/integrals/_two_elec_int.py:293-547 defines it (the engine's other
-// kernels build the same values by the vertical and transfer recursions), :549-812 (horizontal
+// kernels build the same values by vertical recursions), :549-812 (horizontal
 // recursion, component norm), gbasis/base_four_symm.py:195-349 (norm_cont, spherical transform).
 #pragma once
 #include <algorithm>
@@ -259,11 +259,11 @@ __device__ __forceinline__ void rys_sync() {
 // Points of primitive quartets p0, p0 + 1, ... of a quartet with nk ket primitive pairs (kc points,
 // kpp per primitive quartet): lane k writes its point's recursion coefficients PR[.][k], zeros up to a
 // multiple of 4 points.
-template <int N>
-__device__ __forceinline__ void rys_points(const EriLaunch& a, const PrimPair* __restrict__ bprim,
-                                           const PrimPair* __restrict__ kprim, int nk,
+template <class C>
+__device__ __forceinline__ void rys_points(const EriLaunch& a, const PairDev& P, const PairDev& Q,
                                            const double* __restrict__ tab, int p0, int kc, int kpp,
                                            int lane, double* __restrict__ PR) {
+  constexpr int N = C::kN;
   if (lane >= ((kc + 3) & ~3)) return;
   double* const pr = PR + lane;
   if (lane >= kc) {
@@ -272,8 +272,15 @@ __device__ __forceinline__ void rys_points(const EriLaunch& a, const PrimPair* _
     return;
   }
   const int pi = kpp == N ? lane / N : lane / (2 * N), r2 = lane - pi * kpp, r = r2 < N ? r2 : r2 - N;
-  const int ip = (p0 + pi) / nk, jq = p0 + pi - ip * nk;
-  const PrimPair bp = bprim[ip], kp = kprim[jq];
+  const int nk = Q.nprim, ip = (p0 + pi) / nk, jq = p0 + pi - ip * nk;
+  PrimPair bp = a.prims[P.prim_off + ip], kp = a.prims[Q.prim_off + jq];
+  // a flipped pair's recursion centre is its second shell: P - B = (P - A) + (A - B)
+  if constexpr (C::LB == 0 && C::LA > 0) {
+    if (a.flip & 1) { bp.Xx += P.ABx; bp.Xy += P.ABy; bp.Xz += P.ABz; }
+  }
+  if constexpr (C::LD == 0 && C::LC > 0) {
+    if (a.flip & 2) { kp.Xx += Q.ABx; kp.Xy += Q.ABy; kp.Xz += Q.ABz; }
+  }
   const double rs = rsqrt(bp.zeta + kp.zeta), inv = rs * rs;
   const double PQx = bp.Px - kp.Px, PQy = bp.Py - kp.Py, PQz = bp.Pz - kp.Pz;
   const double rz = kp.zeta * inv, re = bp.zeta * inv;  // rho / zeta, rho / eta
@@ -339,7 +346,9 @@ __global__ void __launch_bounds__(32 * C::kW, RysDims<C>::kMinCtas) eri_rys(cons
     const PairDev& Q = a.pairs[pq.y];
     for (int i = tid; i < 4 * kMaxCart; i += NT) {
       const int q = i / kMaxCart, c = i - q * kMaxCart;
-      const ShellDev& s = a.shells[q == 0 ? P.shA : q == 1 ? P.shB : q == 2 ? Q.shA : Q.shB];
+      const bool second = (q & 1) ^ ((a.flip >> (q >> 1)) & 1);
+      const PairDev& pr = q < 2 ? P : Q;
+      const ShellDev& s = a.shells[second ? pr.shB : pr.shA];
       S.scl[q][c] = s.scl[c];
       S.pos[q][c] = s.pos[c];
       if (c == 0) {
@@ -348,9 +357,7 @@ __global__ void __launch_bounds__(32 * C::kW, RysDims<C>::kMinCtas) eri_rys(cons
         S.nint[q] = schwarz ? ncart(s.l) : internal_count(s);
       }
     }
-    const int nbp = P.nprim, nkp = Q.nprim, np = nbp * nkp;
-    const PrimPair* __restrict__ bprim = a.prims + P.prim_off;
-    const PrimPair* __restrict__ kprim = a.prims + Q.prim_off;
+    const int np = P.nprim * Q.nprim;
     double acc[C::kAcc];
 #pragma unroll
     for (int i = 0; i < C::kAcc; ++i) acc[i] = 0.0;
@@ -372,7 +379,7 @@ __global__ void __launch_bounds__(32 * C::kW, RysDims<C>::kMinCtas) eri_rys(cons
       // a chunk per warp, the last warp first (its share of the sums is the lightest): the points'
       // latency (pair data, then table rows at T) is paid once per NW chunks
       const int mine = NW - 1 - wq, p0 = s0 + mine * per_chunk;
-      rys_points<N>(a, bprim, kprim, nkp, tab, p0, min(max(np - p0, 0), per_chunk) * kpp, kpp, lane,
+      rys_points<C>(a, P, Q, tab, p0, min(max(np - p0, 0), per_chunk) * kpp, kpp, lane,
                     PR + mine * kRysRows * kRysKS);
       const int nc = min(NW, (np - s0 + per_chunk - 1) / per_chunk);
       auto padded = [&](int c) {

@@ -299,7 +299,7 @@ def electron_repulsion_integral(basis, transform=None, notation="physicist", *, 
     notation by default (a ``transpose(0, 2, 1, 3)`` view of the chemist array).
 
     ``precision="mixed"`` selects the mixed form: quartets whose final-value Schwarz bound is
-    below ``mixed_skip`` are zero, those below ``mixed_fp32`` run their vertical and transfer
+    below ``mixed_skip`` are zero, those below ``mixed_fp32`` run their vertical
     recursions in FP32.  ``potential`` ("coulomb", "erf" or "erfc", with ``omega``) selects the
     operator, as ``get_boys_function`` does for the reference's integral classes."""
     if notation not in ["physicist", "chemist"]:
