@@ -39,16 +39,22 @@ STREAMS = (1, 2, 4, 6, 8, 12, 16)
 VARIANTS = (0,)
 
 
+# register classes beyond the limit below, after the swap (gen_eri.is_register)
+_LARGER = {(3, 0, 2, 0), (3, 1, 1, 0), (3, 0, 1, 1), (2, 2, 1, 0), (1, 3, 1, 0), (3, 3, 0, 0)}
+
+
 def light_class(cls4):
     """Classes run by the register kernel (the only ones whose team matters): the [e0|f0]
     accumulators and the (ab|cd) block of one quartet fit one thread (170 doubles, the limit
-    the kernel generator uses)."""
+    the kernel generator uses), or, with an s shell's pair run on its other shell, one of six
+    larger ones."""
     def nc(l):
         return (l + 1) * (l + 2) // 2
     la, lb, lc, ld = cls4
     ne = sum(nc(e) for e in range(la, la + lb + 1))
     nf = sum(nc(f) for f in range(lc, lc + ld + 1))
-    return ne * nf + nc(la) * nc(lb) * nc(lc) * nc(ld) <= 170
+    swapped = ((la, lb) if la else (lb, la)) + ((lc, ld) if lc else (ld, lc))
+    return ne * nf + nc(la) * nc(lb) * nc(lc) * nc(ld) <= 170 or swapped in _LARGER
 
 
 def cache_path():

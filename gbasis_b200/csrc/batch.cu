@@ -160,20 +160,6 @@ struct UploadSet {
   }
 };
 
-// Lanes per quartet of the register kernel: about four primitive quartets per lane, fewer
-// lanes when the accumulator set (reduced by shuffles) is large.
-static int default_team(int cb, int ck, double avg_prims) {
-  const int la = kPairClassL[cb][0], lb = kPairClassL[cb][1];
-  const int lc = kPairClassL[ck][0], ld = kPairClassL[ck][1];
-  int ne = 0, nf = 0;
-  for (int e = la; e <= la + lb; ++e) ne += ncart(e);
-  for (int f = lc; f <= lc + ld; ++f) nf += ncart(f);
-  const int cap = ne * nf > 100 ? 2 : (ne * nf > 40 ? 8 : 32);
-  int t = 1;
-  while (t < cap && avg_prims / (2 * t) >= 4.0) t *= 2;
-  return t;
-}
-
 static int build_batch(Batch& Bt, int n_mol, const int* mol_nshells, const int* angmom,
                        const int* nprim, const double* center, const double* exps,
                        const double* coefs, const int* nout, const int* sph, const int8_t* pos,

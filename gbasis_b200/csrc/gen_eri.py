@@ -449,6 +449,22 @@ def is_light(c):
     return ne * nf + ncart(la) * ncart(lb) * ncart(lc) * ncart(ld) <= LIGHT_LIMIT
 
 
+def is_register(c):
+    """Classes the register kernel runs: the light ones, and those whose kernel class holds up to
+    102 accumulators raised by up to 600 operations ((fs|ds), (fp|ps), (fs|pp), (dd|ps), (pf|ps),
+    (ff|ss) and the classes that flip to them).  Register against quadrature kernel on 8,000 to
+    160,000 quartets: (sf|sd) 0.51 against 1.20 ms, (sf|pp) 0.46 and 1.18, (dd|sp) 0.68 and 1.33,
+    (pf|sp) 0.85 and 1.41.  Beyond, the recursion's values spill at every primitive quartet: (pd|ds)
+    (114, 723) 3.0 and 2.4 ms, (dp|ds) (96, 723) 0.36 and 0.28, (fs|fs) (100, 1296) 0.59 and 0.40,
+    (dd|ds) (186, 1446) 3.7 and 1.1.  Lists of a hundred quartets lose 0.01 to 0.02 ms; the rule
+    does not look at the list, on which a quartet's value must not depend."""
+    if is_light(c):
+        return True
+    k = kernel_class(c)[0]
+    acc = len(comps_range(k[0], k[0] + k[1])) * len(comps_range(k[2], k[2] + k[3]))
+    return acc <= 102 and sum(k) <= 6 and best_vertical(*k).op_count() <= 600
+
+
 # Largest total angular momentum for which the straight-line register code is emitted: the CPU
 # tests execute it against the oracle for every class up to L = 8, and the device compiles it
 # for classes up to L = 6 only (light classes and the (ab|ss) structs).  Executed on the CPU, the
@@ -505,7 +521,7 @@ def emit_all(lmax, classes=None):
 
 
 def emit_sources(outdir, lmax):
-    """Write eri_gen.cuh (light classes), their instantiation files, the cooperative programs
+    """Write eri_gen.cuh (register classes), their instantiation files, the cooperative programs
     of the heavy classes (coop_programs.cuh) and the class dispatch."""
     import os
     import gen_coop
@@ -520,22 +536,22 @@ def emit_sources(outdir, lmax):
     every = canonical_classes(lmax)
     light = [c for c in every if is_light(c)]
     heavy = [c for c in every if not is_light(c)]
-    light_k = sorted({kernel_class(c)[0] for c in light})
-    heavy_k = sorted({kernel_class(c)[0] for c in heavy})
+    reg_k = sorted({kernel_class(c)[0] for c in every if is_register(c)})
+    rys_k = sorted({kernel_class(c)[0] for c in every if not is_register(c)})
     # the point-charge kernel uses the (ab|ss) structs of every pair class, heavy ones included
     one_e = [(la, lb, 0, 0) for la in range(lmax + 1) for lb in range(lmax + 1)]
-    put("eri_gen.cuh", emit_all(lmax, light_k + [c for c in one_e if c not in light_k]))
+    put("eri_gen.cuh", emit_all(lmax, reg_k + [c for c in one_e if c not in reg_k]))
     # heavy classes first (their cooperative kernels index the table by position), then the
     # light classes, whose programs only the multi-class queue kernel runs
     gen_coop.emit(heavy + light, os.path.join(outdir, "coop_programs.cuh"), n_heavy=len(heavy))
     files = []
-    # spread the light classes over translation units of similar compile cost (code size)
+    # spread the register classes over translation units of similar compile cost (code size)
     nbins = 12
     bins = [[] for _ in range(nbins)]
     load = [0] * nbins
     cost = {c: best_vertical(*c).op_count() + 4 * ncart(c[0]) * ncart(c[1]) * ncart(c[2]) * ncart(c[3])
-            for c in light_k}
-    for c in sorted(light_k, key=lambda c: -cost[c]):
+            for c in reg_k}
+    for c in sorted(reg_k, key=lambda c: -cost[c]):
         k = load.index(min(load))
         bins[k].append(c)
         load[k] += cost[c]
@@ -563,7 +579,7 @@ def emit_sources(outdir, lmax):
     lfiles, launchers = gen_lines.emit_sources(outdir, heavy)
     files += lfiles
     import gen_rys
-    rfiles, rlaunchers = gen_rys.emit_sources(outdir, heavy_k)
+    rfiles, rlaunchers = gen_rys.emit_sources(outdir, rys_k)
     files += rfiles
     lines = ["// Generated by gen_eri.py: (la,lb,lc,ld) -> class kernel launcher.",
              "#include <cstdlib>",
@@ -573,14 +589,15 @@ def emit_sources(outdir, lmax):
              "namespace gbx {",
              "template <int LA, int LB, int LC, int LD>",
              "int launch_t(const EriLaunch& a, int grid, cudaStream_t st);"]
-    for c in light_k:
+    for c in reg_k:
         lines.append(f"extern template int launch_t<{c[0]}, {c[1]}, {c[2]}, {c[3]}>(const EriLaunch&, "
                      "int, cudaStream_t);")
     for c in heavy:
         lines.append(f"int {launchers[c]}(const EriLaunch& a, cudaStream_t st);")
-    for c in heavy_k:
+    for c in rys_k:
         lines.append(f"int {rlaunchers[c]}(const EriLaunch& a, cudaStream_t st);")
-    lines.append("// Heavy classes run the quadrature kernel (eri_rys).  The block's variant knob selects the")
+    lines.append("// Heavy classes run the quadrature kernel (eri_rys) or, the smallest of them, the register kernel")
+    lines.append("// (is_register in gen_eri.py); for both the block's variant knob selects the")
     lines.append("// line kernel (1) or (2) its group form or, for the classes that have one, the split kernel:")
     lines.append("// a thread per quartet, which is faster on long lists of quartets with equal primitive")
     lines.append("// counts (33,000 to 120,000 quartets of 45 to 60 primitive quartets: 1.4 to 1.8 times,")
@@ -602,14 +619,18 @@ def emit_sources(outdir, lmax):
     lines.append("  EriLaunch a = args;")
     lines.append("  a.flip = (la == 0 && lb > 0 ? 1 : 0) + (lc == 0 && ld > 0 ? 2 : 0);")
     lines.append("  switch (((la * 8 + lb) * 8 + lc) * 8 + ld) {")
+
+    def main(c):
+        k = kernel_class(c)[0]
+        return "launch_t<%d, %d, %d, %d>(a, grid, st)" % k if is_register(c) \
+            else f"{rlaunchers[k]}(a, st)"
     for c in light:
         key = ((c[0] * 8 + c[1]) * 8 + c[2]) * 8 + c[3]
-        k = kernel_class(c)[0]
-        lines.append(f"    case {key}: return launch_t<{k[0]}, {k[1]}, {k[2]}, {k[3]}>(a, grid, st);")
+        lines.append(f"    case {key}: return {main(c)};")
     for j, c in enumerate(heavy):
         key = ((c[0] * 8 + c[1]) * 8 + c[2]) * 8 + c[3]
         lines.append(f"    case {key}: return heavy_interp() ? launch_coop({j}, a, st) : "
-                     f"a.variant == 0 ? {rlaunchers[kernel_class(c)[0]]}(a, st) : {launchers[c]}(a, st);")
+                     f"a.variant == 0 ? {main(c)} : {launchers[c]}(a, st);")
     lines.append("    default: break;")
     lines.append("  }")
     lines.append('  return set_error(GBX_ERR_UNSUPPORTED, "no kernel for class (%d %d|%d %d)", '

@@ -513,23 +513,13 @@ int build_basis(Basis& B, int n, const int* angmom, const int* nprim, const doub
         }
       }
   }
-  // default lanes-per-quartet: about four primitive quartets per lane, fewer lanes when the
-  // accumulator set (reduced across the team by shuffles) is large
   std::vector<double> cprims(kNumPairClasses, 0.0);
   for (const PairDev& p : B.pairs) cprims[p.cls] += p.nprim;
   for (int c = 0; c < kNumPairClasses; ++c)
     if (B.class_count[c]) cprims[c] /= (double)B.class_count[c];
   for (HostBlock& h : B.blocks) {
     h.avg_prims = cprims[h.cb] * cprims[h.ck];
-    const int la = kPairClassL[h.cb][0], lb = kPairClassL[h.cb][1];
-    const int lc = kPairClassL[h.ck][0], ld = kPairClassL[h.ck][1];
-    int ne = 0, nf = 0;
-    for (int e = la; e <= la + lb; ++e) ne += ncart(e);
-    for (int f = lc; f <= lc + ld; ++f) nf += ncart(f);
-    const int cap = ne * nf > 100 ? 2 : (ne * nf > 40 ? 8 : 32);
-    int t = 1;
-    while (t < cap && h.avg_prims / (2 * t) >= 4.0) t *= 2;
-    h.team = t;
+    h.team = default_team(h.cb, h.ck, h.avg_prims);
   }
   // launch order: estimated work, largest first
   std::vector<double> cost(B.blocks.size());

@@ -68,6 +68,24 @@ int boys_table(int device, const double** out);
 int rys_table(const double** out);  // quadrature points and weights on the current device
 int compiled_lmax();
 
+// Lanes per quartet of the register kernel: about four primitive quartets per lane, fewer lanes
+// when the accumulator set of the class's kernel (reduced by shuffles) is large.  Above 50
+// accumulators 4 lanes at most: 2 or 4 are the best on 8,000 and more quartets of 38 to 72 primitive
+// quartets ((sf|pp) 0.458 and 0.472 ms, 8 lanes 0.568; (dd|sp) 0.679 and 0.683, 0.799).
+inline int default_team(int cb, int ck, double avg_prims) {
+  int n = 1;
+  for (const int c : {cb, ck}) {
+    const int a = kPairClassL[c][0], b = kPairClassL[c][1];
+    int m = 0;  // an s shell's pair runs on its other shell: [l0| alone
+    for (int e = a ? a : b; e <= a + b; ++e) m += ncart(e);
+    n *= m;
+  }
+  const int cap = n > 100 ? 2 : n > 50 ? 4 : n > 40 ? 8 : 32;
+  int t = 1;
+  while (t < cap && avg_prims / (2 * t) >= 4.0) t *= 2;
+  return t;
+}
+
 // Diagonal blocks whose quartets run from the better-conditioned pair (quartet_transposed):
 // those of pairs with lA + lB >= 3, where a contracted recursion run from a poorly placed
 // centre loses digits; the lighter ones keep one orientation (no divergent stores).

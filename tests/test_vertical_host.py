@@ -7,6 +7,7 @@ import sys
 import numpy as np
 import pytest
 
+from gbasis_b200.autotune import light_class
 from gbasis_b200.contractions import GeneralizedContractionShell
 from oracle import eri_oracle as orc
 
@@ -16,7 +17,7 @@ sys.path.insert(0, CSRC)
 import gen_eri  # noqa: E402
 
 EVERY = gen_eri.canonical_classes(3)
-LIGHT = [c for c in EVERY if gen_eri.is_light(c)]
+REGISTER = [c for c in EVERY if gen_eri.is_register(c)]
 
 
 def _run(emit, env):
@@ -35,11 +36,13 @@ def test_kernel_classes():
         assert not (k[0] == 0 < k[1]) and not (k[2] == 0 < k[3])
         assert gen_eri.kernel_class(k) == (k, 0)
         if gen_eri.is_light(c):
-            assert gen_eri.is_light(k) and sum(k) <= gen_eri.MAX_EMIT_L
+            assert gen_eri.is_light(k) and gen_eri.is_register(c)
+        assert gen_eri.is_register(c) == gen_eri.is_register(k) == light_class(c)
+        assert not gen_eri.is_register(c) or sum(k) <= gen_eri.MAX_EMIT_L
 
 
 @pytest.mark.parametrize("tight", [False, True])
-@pytest.mark.parametrize("cls", LIGHT)
+@pytest.mark.parametrize("cls", REGISTER)
 def test_vertical_recursion_matches_oracle(cls, tight):
     """`tight`: s shells of exponent 40 far from their partners, so that a flipped pair's centre is
     far from P.  Values of order 1 at most; 1e-12 absolute as for the engine."""
