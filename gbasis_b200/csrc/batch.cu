@@ -266,7 +266,22 @@ static int build_batch(Batch& Bt, int n_mol, const int* mol_nshells, const int* 
   up.add(&Bt.d_pairs, pairs);
   up.add(&Bt.d_exps, hexps);
   up.add(&Bt.d_coefs, hcoefs);
-  if ((s = Bt.upload(&Bt.d_work, work, "upload batch work list"))) return s;
+  // the list as built goes to the compact store (scratch here: a quartet has at least one element
+  // there), from where order_work puts it in order
+  static_assert(sizeof(int2) == sizeof(double), "work list in the compact store");
+  if ((s = Bt.alloc((void**)&Bt.d_work, work.size() * sizeof(int2), "cudaMalloc(batch work list)")))
+    return s;
+  if ((s = Bt.alloc((void**)&Bt.d_compact, (size_t)Bt.compact_elems * sizeof(double),
+                    "cudaMalloc(batch compact store)")))
+    return s;
+  if ((long long)work.size() > Bt.compact_elems)
+    return set_error(GBX_ERR_INVALID, "batch work list larger than its compact store");
+  GBX_CUDA(cudaMemcpy(Bt.d_compact, work.data(), work.size() * sizeof(int2), cudaMemcpyHostToDevice),
+           "upload batch work list");
+  std::vector<ListSegment> segs;
+  for (const BatchType& T : Bt.types) segs.push_back({T.work_off, T.n});
+  ListSegment* d_segs = nullptr;
+  up.add(&d_segs, segs);
   Bt.h_work = std::move(work);
   Bt.pair_off = pair_off;
   if ((s = Bt.alloc((void**)&Bt.d_prims, (size_t)std::max<long long>(pp0, 1) * sizeof(PrimPair),
@@ -278,9 +293,6 @@ static int build_batch(Batch& Bt, int n_mol, const int* mol_nshells, const int* 
     up.add(&Bt.types[k].d_base, tbase[k]);
     up.add(&Bt.types[k].d_ncols, tcols[k]);
   }
-  if ((s = Bt.alloc((void**)&Bt.d_compact, (size_t)Bt.compact_elems * sizeof(double),
-                    "cudaMalloc(batch compact store)")))
-    return s;
 
   // expansion tables and descriptors
   std::vector<int> gtab;
@@ -309,6 +321,9 @@ static int build_batch(Batch& Bt, int n_mol, const int* mol_nshells, const int* 
   pair_precompute<<<(np + 127) / 128, 128>>>(Bt.d_pairs, np, Bt.d_shells, Bt.d_exps, Bt.d_coefs,
                                              Bt.d_prims);
   GBX_CUDA(cudaGetLastError(), "pair_precompute launch");
+  order_work<<<(int)segs.size(), kOrderThreads>>>(d_segs, (const int2*)Bt.d_compact, Bt.d_pairs,
+                                                  Bt.d_work);
+  GBX_CUDA(cudaGetLastError(), "order_work launch");
   if ((s = alloc_fault_word(&Bt.d_fault))) return s;
   if (Bt.d_fault) Bt.allocs.push_back({Bt.d_fault, sizeof(unsigned long long)});
   Bt.h_exp.resize(n_mol);

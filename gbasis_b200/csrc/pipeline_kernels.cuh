@@ -41,6 +41,14 @@ __global__ void pair_precompute(PairDev* __restrict__ pairs, int npairs,
                                 const ShellDev* __restrict__ shells,
                                 const double* __restrict__ exps, const double* __restrict__ coefs,
                                 PrimPair* __restrict__ prims);
+// One list of quartets: entries [off, off + n).
+struct ListSegment {
+  long long off, n;
+};
+constexpr int kOrderThreads = 1024, kOrderBuckets = 128;
+// dst[off..off + n) = the quartets of src there, most primitive quartets first (a CTA per segment).
+__global__ void order_work(const ListSegment* __restrict__ segs, const int2* __restrict__ src,
+                           const PairDev* __restrict__ pairs, int2* __restrict__ dst);
 // Mixed form of the work-list build (counts32 == nullptr: FP64 only, nothing skipped).
 struct MixedParams {
   const double* qm;  // per pair: Schwarz bound x largest output scale of its two shells
