@@ -562,7 +562,7 @@ def main():
     compute_tf = flops / (ph[1] * 1e-3) / 1e12
     exp_bytes = 8.0 * n ** 4 + compact_bytes  # tensor written + compact store read once
     exp_gbs = exp_bytes / (ph[2] * 1e-3) / 1e9
-    roof_compute = {"kernel": "class kernels (eri_block, eri_split, eri_lines; all class blocks, concurrent)", "bound": "fp64", "achieved": compute_tf,
+    roof_compute = {"kernel": "class kernels (eri_block, eri_rys; all class blocks, concurrent)", "bound": "fp64", "achieved": compute_tf,
                     "peak": peak64, "unit": "TFLOP/s", "frac": compute_tf / peak64,
                     "peak_source": "gbx_fp64_peak dependent-FMA probe, measured live",
                     "traffic": None, "ms": ph[1], "algorithmic_flops": flops}
