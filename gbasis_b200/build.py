@@ -43,12 +43,12 @@ def sources(lmax):
     import gen_eri  # noqa: E402
     gen = gen_eri.emit_sources(GEN, lmax)
     return [os.path.join(GEN, g) for g in gen] + [
-        os.path.join(CSRC, f) for f in ("runtime.cu", "pipeline.cu", "extras.cu", "noalloc.cu",
+        os.path.join(CSRC, f) for f in ("runtime.cu", "pools.cu", "pipeline.cu", "extras.cu", "noalloc.cu",
                                         "coop_kernel.cu", "batch.cu", "one_elec.cu", "boys_eval.cu")]
 
 
 KERNEL_DEPS = ("gbx_common.cuh", "eri_kernels.cuh", "errors.h", "_gen/eri_gen.cuh")
-HOST_DEPS = ("gbx_common.cuh", "runtime.h", "errors.h", "pipeline_kernels.cuh", "coop.cuh",
+HOST_DEPS = ("gbx_common.cuh", "runtime.h", "pools.h", "errors.h", "pipeline_kernels.cuh", "coop.cuh",
              "coop_tail.cuh", "_gen/coop_programs.cuh")
 
 

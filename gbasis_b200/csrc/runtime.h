@@ -10,6 +10,7 @@
 #include "errors.h"
 #include "gbx_common.cuh"
 #include "gbx_eri.h"
+#include "pools.h"
 
 namespace gbx {
 
@@ -33,36 +34,11 @@ constexpr int kMaxAuxStreams = 16;  // the most a basis may be given
 constexpr long long kMinFp32List = 65536;
 constexpr long long kFp32ListShare = 4;
 constexpr long long kCoulombChunk = 1LL << 23;  // quartets per direct-Coulomb work chunk
-constexpr int kStageBuffers = 3;                // host-output staging slabs in flight
 constexpr size_t kStageBytes = 64ull << 20;     // target bytes of one staging slab
 constexpr size_t kStageSlabs = 8;               // least number of slabs of a tensor above 16 MB
 // Pageable tensors up to this size are copied out of the ring by the calling thread: starting and
 // joining the copy threads takes about 0.25 ms, what one thread copies in that time
 constexpr size_t kOneThreadCopy = 2ull << 20;
-
-// Streams and events of one basis or batch: the class blocks' auxiliary streams, their join and fork
-// events, and the host-output copy stream with the staging slabs' events.  Sets live in a pool per
-// device (streams_take / streams_give): creating and destroying 7 streams and 13 events took 2 of
-// the 2.9 ms of a 20-function host call.  A set has one owner at a time.
-struct StreamSet {
-  int device = 0;
-  std::vector<cudaStream_t> aux;
-  std::vector<cudaEvent_t> join;
-  cudaEvent_t fork = nullptr, in = nullptr, out = nullptr;
-  cudaStream_t copy = nullptr;
-  cudaEvent_t stage_ready[kStageBuffers] = {};
-  cudaEvent_t stage_free[kStageBuffers] = {};
-  int ensure_aux(int n);  // at least n auxiliary streams
-  ~StreamSet();
-};
-// A set for the current device (from the pool, or a new one).
-int streams_take(int device, std::unique_ptr<StreamSet>* out);
-// Back to the pool, or destroyed when the pool is full; the caller has made sure that no work is
-// queued on its streams (idle), else the set is destroyed.
-void streams_give(std::unique_ptr<StreamSet> set, bool idle);
-// Device blocks of the process's block cache (gbx_release_cached_memory empties it).
-int block_alloc(int device, void** p, size_t bytes, size_t* got, const char* what);
-void block_give(int device, void* p, size_t bytes);  // no work on the device still uses p
 
 int boys_table(int device, const double** out);
 int rys_table(const double** out);  // quadrature points and weights on the current device
