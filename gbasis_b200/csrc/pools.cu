@@ -18,7 +18,8 @@ namespace gbx {
 // kBlockCacheBytes per device: the public full-tensor call builds and drops a basis every time,
 // and cudaFree (which waits for the whole device) plus cudaMalloc of the compact store and the
 // staging slabs cost milliseconds per call.  A block is reused for a request of at least half
-// its size.  gbx_release_cached_memory() frees the cache.
+// its size.  gbx_release_cached_memory() frees the cache, and so does an allocation that finds the
+// device full: what would fit without the cache fits with it.
 constexpr size_t kBlockCacheBytes = size_t(2) << 30;
 struct CachedBlock {
   int device;
@@ -58,11 +59,34 @@ void block_give(int device, void* p, size_t bytes) {
   cudaFree(p);
 }
 
+// Frees the idle blocks of a device (of all: device < 0); whether there were any.
+static bool cache_drop(int device) {
+  std::vector<CachedBlock> drop;
+  {
+    std::lock_guard<std::mutex> lk(g_block_mu);
+    for (size_t i = g_blocks.size(); i-- > 0;)
+      if (device < 0 || g_blocks[i].device == device) {
+        drop.push_back(g_blocks[i]);
+        g_blocks.erase(g_blocks.begin() + i);
+      }
+  }
+  for (const CachedBlock& b : drop) {
+    DeviceGuardLite g(b.device);
+    cudaFree(b.p);
+  }
+  return !drop.empty();
+}
+
 int block_alloc(int device, void** p, size_t bytes, size_t* got, const char* what) {
   if (bytes == 0) bytes = 16;
   *p = cache_take(device, bytes, got);
   if (!*p) {
-    GBX_CUDA(cudaMalloc(p, bytes), what);
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation && cache_drop(device)) {
+      cudaGetLastError();  // the failed attempt's error
+      e = cudaMalloc(p, bytes);
+    }
+    GBX_CUDA(e, what);
     *got = bytes;
   }
   return GBX_OK;
@@ -133,17 +157,12 @@ void streams_give(std::unique_ptr<StreamSet> set, bool idle) {
 }
 
 void release_pools() {
-  std::vector<CachedBlock> blocks;
   std::vector<std::unique_ptr<StreamSet>> sets;  // destroyed at the end, outside the lock
   {
     std::lock_guard<std::mutex> lk(g_block_mu);
-    blocks.swap(g_blocks);
     sets.swap(g_stream_sets);
   }
-  for (const CachedBlock& b : blocks) {
-    DeviceGuardLite g(b.device);
-    cudaFree(b.p);
-  }
+  cache_drop(-1);
 }
 
 }  // namespace gbx

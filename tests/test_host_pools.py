@@ -92,3 +92,26 @@ def test_a_set_stays_usable_after_a_failed_event(tmp_path):
   s.reset();
   CHECK(streams == 0 && events == 0);
 """)
+
+
+def test_a_full_device_takes_the_idle_blocks(tmp_path):
+    """An allocation that fits without the cache's idle blocks succeeds, leaves no error behind and
+    frees them; one that does not fit fails as before, and blocks in use stay."""
+    _run(tmp_path, r"""
+  capacity = 1000;
+  void *a, *b, *c;
+  size_t na, nb, nc;
+  CHECK(block_alloc(0, &a, 300, &na, "a") == GBX_OK && na == 300);
+  CHECK(block_alloc(0, &b, 500, &nb, "b") == GBX_OK);
+  block_give(0, b, nb);  // idle: 500 of the 800 in use
+  CHECK(block_alloc(0, &c, 600, &nc, "c") == GBX_OK && nc == 600);
+  CHECK(cudaGetLastError() == cudaSuccess && used == 900);
+  block_give(0, c, nc);
+  CHECK(block_alloc(0, &b, 900, &nb, "b") == GBX_ERR_OOM);
+  CHECK(used == 300 && blocks.count(a));
+  block_give(0, a, na);
+  CHECK(block_alloc(0, &b, 200, &nb, "b") == GBX_OK && b == a && nb == 300);  // reused
+  block_give(0, b, nb);
+  release_pools();
+  CHECK(used == 0);
+""")
