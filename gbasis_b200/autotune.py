@@ -18,7 +18,9 @@ the block types of a batch.  Choices are stored in a JSON cache keyed by class a
 the block's mean primitive quartets per shell quartet (team: ``"abcd:k"``, variant:
 ``"v:abcd:k"``, grid cap: ``"c:abcd:k"``; stream count: ``"streams"``), so a new basis or
 batch of similar shape starts tuned (``DeviceBasis`` and ``EriBatch`` apply the cache on
-creation).  gbasis has no counterpart: it evaluates one quartet at a time in NumPy.
+creation).  The file names the generation of the kernels that it was measured on (``KERNELS``): a
+file of another generation, or of none, is not used.  gbasis has no counterpart: it evaluates one
+quartet at a time in NumPy.
 """
 from __future__ import annotations
 
@@ -37,6 +39,11 @@ TEAMS = (1, 2, 4, 8, 16, 32)
 CTAS = (2, 4, 8, 16)
 STREAMS = (1, 2, 4, 6, 8, 12, 16)
 VARIANTS = (0,)
+# Generation of the class kernels: raised when a class changes its kernel, its kernel changes what
+# a knob does or is best at, or a variant number changes its meaning.  1 had no tag: its variant 1
+# was the faster one for many classes that now run 3 to 14 times slower on it than by default, and
+# its lane counts belong to another recursion.
+KERNELS = 2
 
 
 # register classes beyond the limit below, after the swap (gen_eri.is_register)
@@ -83,15 +90,27 @@ def _load():
             return dict(hit[1])
         with open(path) as f:
             table = json.load(f)
+        if table.pop("kernels", None) != KERNELS:
+            table = {}
         _loaded[path] = (mtime, table)
         return dict(table)
     except (OSError, ValueError):
         return {}
 
 
+def _store(chosen):
+    """The cache file with the choices ``chosen``, without entries of another generation and without
+    variants and grid caps that are the default (looked up on every creation for nothing)."""
+    table = {**_load(), **chosen, "kernels": KERNELS}
+    table = {k: v for k, v in table.items()
+             if not (k.startswith("v:") and v == 0 or k.startswith("c:") and v == 8)}
+    with open(cache_path(), "w") as f:
+        json.dump(table, f, indent=1, sort_keys=True)
+
+
 def apply_cache(db, table=None):
-    """Set the knobs of every block whose (class, primitive bucket) the cache knows, and the
-    stream count; returns how many blocks changed."""
+    """Set the knobs of every block whose (class, primitive bucket) the cache (or ``table``, used
+    as it is) knows, and the stream count; returns how many blocks changed."""
     table = _load() if table is None else table
     configs = any(key.startswith(("v:", "c:")) for key in table)
     n = 0
@@ -126,6 +145,14 @@ def _call_ms(db, reps):
     return best
 
 
+def _pick(values, times, current):
+    """The fastest value, or the current one where none is 3 % faster (runs differ by 1 to 2 %)."""
+    values, best = list(values), int(np.argmin(times))
+    if current in values and times[values.index(current)] * 0.97 <= times[best]:
+        return current
+    return values[best]
+
+
 def _sweep(db, blocks, ks, values, setter, reps):
     """Per-block times (values x blocks) of each value of one knob, blocks run in order."""
     times = np.full((len(values), len(blocks)), np.inf)
@@ -155,7 +182,7 @@ def autotune(shells, coord_types=None, reps=3, teams=TEAMS, ctas=CTAS, streams=S
     # lanes per quartet (light classes)
     t_team = _sweep(db, blocks, light, teams, db.set_team, reps)
     for k in light:
-        best = teams[int(np.argmin(t_team[:, k]))]
+        best = _pick(teams, t_team[:, k], blocks[k][1])
         db.set_team(k, best)
         chosen[keys[k]] = best
     timings["team"] = t_team
@@ -172,12 +199,12 @@ def autotune(shells, coord_types=None, reps=3, teams=TEAMS, ctas=CTAS, streams=S
         db.set_block_config(k, var[k], c)
     t_var = _sweep(db, blocks, heavy, VARIANTS, set_var, reps)
     for k in heavy:
-        set_var(k, VARIANTS[int(np.argmin(t_var[:, k]))])
+        set_var(k, _pick(VARIANTS, t_var[:, k], 0))
         chosen["v:" + keys[k]] = var[k]
     timings["variant"] = t_var
     t_cap = _sweep(db, blocks, light, ctas, set_cap, reps)
     for k in light:
-        set_cap(k, ctas[int(np.argmin(t_cap[:, k]))])
+        set_cap(k, _pick(ctas, t_cap[:, k], 8))
         chosen["c:" + keys[k]] = cap[k]
     timings["ctas_per_sm"] = t_cap
     # stream count, on whole calls with the blocks concurrent
@@ -187,14 +214,11 @@ def autotune(shells, coord_types=None, reps=3, teams=TEAMS, ctas=CTAS, streams=S
         db.set_streams(n)
         db.unique()
         t_st.append(_call_ms(db, reps))
-    chosen["streams"] = streams[int(np.argmin(t_st))]
+    chosen["streams"] = _pick(streams, np.array(t_st), 6)
     db.set_streams(chosen["streams"])
     timings["streams"] = np.array(t_st)
     if save:
-        table = _load()
-        table.update(chosen)
-        with open(cache_path(), "w") as f:
-            json.dump(table, f, indent=1, sort_keys=True)
+        _store(chosen)
     db.close()
     return chosen, timings
 
@@ -217,10 +241,7 @@ def main(argv):
             chosen, _ = autotune(make_workload(name))
             if keep is not None and name != argv[0]:
                 # the first single-basis workload sets the stream count
-                table = _load()
-                table["streams"] = keep
-                with open(cache_path(), "w") as f:
-                    json.dump(table, f, indent=1, sort_keys=True)
+                _store({"streams": keep})
         print(name, json.dumps(chosen, sort_keys=True), flush=True)
 
 

@@ -101,8 +101,7 @@ class EriBatch:
         CUDA events per type): the team of the register-kernel types, then the kernel variant
         of the heavy types, then the grid cap of the register-kernel types; keep the fastest
         and store the choices in the tuning cache."""
-        import json
-        from .autotune import CTAS, TEAMS, VARIANTS, _key, _load, cache_path, light_class
+        from .autotune import CTAS, TEAMS, VARIANTS, _key, _pick, _store, light_class
         teams = TEAMS if teams is None else teams
         L = _engine.lib()
         types = self.types()
@@ -136,25 +135,22 @@ class EriBatch:
         try:
             times = sweep(light, teams, self.set_team)
             for k in light:
-                best = teams[int(np.argmin(times[:, k]))]
+                best = _pick(teams, times[:, k], types[k][1])
                 self.set_team(k, best)
                 chosen[keys[k]] = best
             t_var = sweep(heavy, VARIANTS, set_var)
             for k in heavy:
-                set_var(k, VARIANTS[int(np.argmin(t_var[:, k]))])
+                set_var(k, _pick(VARIANTS, t_var[:, k], 0))
                 chosen["v:" + keys[k]] = var[k]
             t_cap = sweep(light, CTAS, set_cap)
             for k in light:
-                set_cap(k, CTAS[int(np.argmin(t_cap[:, k]))])
+                set_cap(k, _pick(CTAS, t_cap[:, k], 8))
                 chosen["c:" + keys[k]] = cap[k]
         finally:
             _engine.check(L.gbx_batch_set_profiling(self.handle, 0))
         times = {"team": times, "variant": t_var, "ctas_per_sm": t_cap}
         if save:
-            table = _load()
-            table.update(chosen)
-            with open(cache_path(), "w") as f:
-                json.dump(table, f, indent=1, sort_keys=True)
+            _store(chosen)
         return chosen, times
 
     def run(self, outs, notation="chemist", stream=None, mixed=None):
