@@ -74,8 +74,8 @@ struct Batch {
   bool profile = false;
   std::vector<cudaEvent_t> type_ev;
   std::vector<std::pair<void*, size_t>> allocs;
-  // mixed-precision form: the FP64 work list and first merged pair of each molecule kept on
-  // the host; per pair the bound of its output functions; per type, in d_work_mixed, the
+  // mixed-precision form: the FP64 work list (fetched from the device for the first mixed lists)
+  // and first merged pair of each molecule on the host; per pair the bound of its output functions; per type, in d_work_mixed, the
   // FP64 quartets followed by the FP32 ones (quartets below the skip bound left out)
   std::vector<int2> h_work;
   std::vector<long long> pair_off;
@@ -282,7 +282,6 @@ static int build_batch(Batch& Bt, int n_mol, const int* mol_nshells, const int* 
   for (const BatchType& T : Bt.types) segs.push_back({T.work_off, T.n});
   ListSegment* d_segs = nullptr;
   up.add(&d_segs, segs);
-  Bt.h_work = std::move(work);
   Bt.pair_off = pair_off;
   if ((s = Bt.alloc((void**)&Bt.d_prims, (size_t)std::max<long long>(pp0, 1) * sizeof(PrimPair),
                     "cudaMalloc(batch primitive pairs)")))
@@ -457,6 +456,12 @@ static int batch_mixed_lists(Batch& Bt, double skip, double fp32) {
   if (Bt.d_work_mixed && skip == Bt.mix_skip && fp32 == Bt.mix_fp32) return GBX_OK;
   int s;
   if ((s = batch_mixed_bounds(Bt))) return s;
+  if (Bt.h_work.empty()) {  // in the order of the FP64 form: parts of ordered lists are ordered
+    std::vector<int2> h((size_t)Bt.n_quartets);
+    GBX_CUDA(cudaMemcpy(h.data(), Bt.d_work, h.size() * sizeof(int2), cudaMemcpyDeviceToHost),
+             "download batch work list");
+    Bt.h_work = std::move(h);
+  }
   const size_t nt = Bt.types.size();
   std::vector<int2> w, w32;
   w.reserve(Bt.h_work.size());

@@ -1,0 +1,43 @@
+"""GPU test of the order of a batch's mixed-form work lists: by primitive quartets, as the FP64 form's.
+
+With nothing left out and nothing in FP32 the mixed form runs the FP64 form's quartets on the same
+kernels, so that equal orders take equal times; lists in the order of the molecules take about twice
+as long on the molecules below, whose neighbouring quartets differ by up to 1,296 times in length.
+The bar of 1.25 allows for the spread of best-of-many times.
+"""
+import numpy as np
+import pytest
+
+from gbasis_b200.batch import EriBatch
+from gbasis_b200.contractions import GeneralizedContractionShell
+
+pytestmark = pytest.mark.gpu
+
+
+def _molecule(rng):
+    return [GeneralizedContractionShell(1, rng.uniform(-1.5, 1.5, 3), rng.uniform(0.2, 1.0, k),
+                                        0.4 * 1.6 ** np.arange(k), "cartesian")
+            for k in (6, 1, 6, 1)]
+
+
+def test_mixed_lists_run_in_the_order_of_the_fp64_lists():
+    import torch
+    rng = np.random.default_rng(5)
+    b = EriBatch([_molecule(rng) for _ in range(1500)])
+    outs = [[torch.zeros((n,) * 4, dtype=torch.float64, device="cuda") for n in b.nbf] for _ in range(2)]
+    forms = (None, (0.0, 0.0))
+    best = [np.inf, np.inf]
+    for rep in range(12):
+        for i, mixed in enumerate(forms):
+            e0, e1 = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            e0.record()
+            b.run(outs[i], mixed=mixed)
+            e1.record()
+            e1.synchronize()
+            if rep > 1:
+                best[i] = min(best[i], e0.elapsed_time(e1))
+    assert b.mixed_counts()[1:] == (0, 0)
+    for x, y in zip(*outs):
+        assert torch.equal(x, y)
+    b.close()
+    assert best[1] <= 1.25 * best[0], best
