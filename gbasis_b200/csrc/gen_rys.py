@@ -20,6 +20,7 @@ warps of a CTA.  ``root_tables`` makes the points and weights as piecewise polyn
 from __future__ import annotations
 
 import functools
+import hashlib
 import itertools
 import math
 import os
@@ -407,7 +408,11 @@ def emit_sources(outdir, classes, nfiles=12):
         _put(os.path.join(outdir, name), "\n".join(out) + "\n")
         files.append(name)
     path = os.path.join(outdir, "rys_tables.cu")
-    head = f"// Generated by gen_rys.py: points and weights, degree {DEG} on unit intervals, two degrees a row, ranges {TMAX}."
+    # making the table takes seconds: kept while this generator is the one that made it
+    with open(__file__, "rb") as f:
+        made_by = hashlib.sha256(f.read()).hexdigest()[:16]
+    head = (f"// Generated by gen_rys.py ({made_by}): points and weights, degree {DEG} on unit intervals, "
+            f"two degrees a row, ranges {TMAX}.")
     if not (os.path.exists(path) and open(path).readline().rstrip("\n") == head):
         vals = [v for n in TMAX for v in root_table(n)]
         text = "\n".join([
