@@ -495,6 +495,8 @@ static int batch_mixed_lists(Batch& Bt, double skip, double fp32) {
       (s = Bt.alloc((void**)&Bt.d_work_mixed, std::max<size_t>(Bt.h_work.size(), 1) * sizeof(int2),
                     "cudaMalloc(batch mixed work list)")))
     return s;
+  // a run with other thresholds may still be reading the lists
+  GBX_CUDA(cudaStreamSynchronize(Bt.exec), "wait for the last mixed run");
   GBX_CUDA(cudaMemcpy(Bt.d_work_mixed, w.data(), w.size() * sizeof(int2), cudaMemcpyHostToDevice),
            "upload batch mixed work list");
   long long n32 = 0;
