@@ -1056,7 +1056,9 @@ static int ensure_mixed_counts(Basis& B, double skip, double fp32) {
     on[k] = B.mix_n32[k] >= B.fp32_min && B.mix_n32[k] * B.fp32_share >= h.ncand;
     if (!on[k]) B.mix_n32[k] = 0;
   }
-  if (!B.d_fp32_on && B.alloc((void**)&B.d_fp32_on, nblk * sizeof(int), "cudaMalloc(fp32 flags)"))
+  if (B.d_fp32_on)  // a run with other thresholds, on any stream, may still be reading the flags
+    GBX_CUDA(cudaDeviceSynchronize(), "wait for the last mixed run");
+  else if (B.alloc((void**)&B.d_fp32_on, nblk * sizeof(int), "cudaMalloc(fp32 flags)"))
     return GBX_ERR_OOM;
   GBX_CUDA(cudaMemcpy(B.d_fp32_on, on.data(), nblk * sizeof(int), cudaMemcpyHostToDevice),
            "upload fp32 flags");
