@@ -70,17 +70,15 @@ extern "C" int gbx_boys_eval(int m_max, int64_t n, const double* T, double* F) {
   if (s) return s;
   const double* tab = nullptr;
   if ((s = boys_table(dev, &tab))) return s;
-  double *dT = nullptr, *dF = nullptr;
   const size_t nf = (size_t)n * (m_max + 1);
-  if ((s = cuda_status(cudaMalloc(&dT, n * sizeof(double)), "cudaMalloc(T)"))) return s;
-  if ((s = cuda_status(cudaMalloc(&dF, nf * sizeof(double)), "cudaMalloc(F)"))) {
-    cudaFree(dT);
-    return s;
-  }
+  double* dT = nullptr;  // arguments, then values
+  size_t got = 0;
+  if ((s = block_alloc(dev, (void**)&dT, (n + nf) * sizeof(double), &got, "cudaMalloc(T, F)"))) return s;
+  double* dF = dT + n;
   s = cuda_status(cudaMemcpy(dT, T, n * sizeof(double), cudaMemcpyHostToDevice), "upload T");
   if (!s) s = launch_boys<0>(m_max, tab, dT, n, dF, 0);
   if (!s) s = cuda_status(cudaMemcpy(F, dF, nf * sizeof(double), cudaMemcpyDeviceToHost), "download F");
-  cudaFree(dT);
-  cudaFree(dF);
+  if (!s) block_give(dev, dT, got);  // the copy back waited for the kernel
+  else cudaFree(dT);
   return s;
 }

@@ -1686,13 +1686,17 @@ int unique_values(Basis& B, long long n, const long long* idx4_host, double* out
       return set_error(GBX_ERR_INVALID, "function index %lld out of range [0, %lld)",
                        (long long)idx4_host[i], B.nbf);
   if (n == 0) return GBX_OK;
-  long long* d_idx = nullptr;
-  double* d_out = nullptr;
-  GBX_CUDA(cudaMalloc(&d_idx, (size_t)n * 4 * sizeof(long long)), "cudaMalloc(indices)");
-  cudaError_t err = cudaMalloc(&d_out, (size_t)n * sizeof(double));
-  if (err == cudaSuccess)
-    err = cudaMemcpyAsync(d_idx, idx4_host, (size_t)n * 4 * sizeof(long long),
-                          cudaMemcpyHostToDevice, st);
+  // indices and values in one block of the cache: an allocation of its own would not find the
+  // memory that idle blocks hold
+  unsigned char* tmp = nullptr;
+  size_t got = 0;
+  int s = block_alloc(B.device, (void**)&tmp, (size_t)n * (4 * sizeof(long long) + sizeof(double)), &got,
+                      "cudaMalloc(indices)");
+  if (s) return s;
+  long long* d_idx = reinterpret_cast<long long*>(tmp);
+  double* d_out = reinterpret_cast<double*>(d_idx + 4 * n);
+  cudaError_t err = cudaMemcpyAsync(d_idx, idx4_host, (size_t)n * 4 * sizeof(long long),
+                                    cudaMemcpyHostToDevice, st);
   if (err == cudaSuccess) {
     gather_unique<<<(int)((n + 255) / 256), 256, 0, st>>>(expand_args(B, GBX_CHEMIST, nullptr),
                                                         d_idx, n, d_out);
@@ -1701,8 +1705,8 @@ int unique_values(Basis& B, long long n, const long long* idx4_host, double* out
   if (err == cudaSuccess)
     err = cudaMemcpyAsync(out_host, d_out, (size_t)n * sizeof(double), cudaMemcpyDeviceToHost, st);
   if (err == cudaSuccess) err = cudaStreamSynchronize(st);
-  cudaFree(d_idx);
-  if (d_out) cudaFree(d_out);
+  if (err == cudaSuccess) block_give(B.device, tmp, got);  // the stream is idle
+  else cudaFree(tmp);
   return cuda_status(err, "unique values");
 }
 
