@@ -108,16 +108,34 @@ def _store(chosen):
         json.dump(table, f, indent=1, sort_keys=True)
 
 
+# Threads that keep the device busy: 148 SMs of 8 warps, two per scheduler.  Entries as they are,
+# this bound, twice it and four times it: one (dp|ps) quartet 0.60, 0.42, 0.42, 0.43 ms, resident s-f
+# chain of 7 atoms 6.75, 6.87, 6.96, 7.05 ms, 60-molecule batch 12.58, 12.57, 12.63, 12.68 ms.
+FILL = 148 * 256
+
+
+def _lanes(entry, team, quartets):
+    """Lanes per quartet for a block whose rule says ``team`` and whose cache entry is ``entry``: the
+    entry was measured on lists of 49,000 quartets and more, where fewer lanes leave less to add up;
+    a shorter list takes as many more, up to the rule's, as it needs to fill the device."""
+    while entry < team and quartets * entry < FILL:
+        entry *= 2
+    return entry
+
+
 def apply_cache(db, table=None):
-    """Set the knobs of every block whose (class, primitive bucket) the cache (or ``table``, used
-    as it is) knows, and the stream count; returns how many blocks changed."""
+    """Set the knobs of every block whose (class, primitive bucket) the cache knows (lanes as
+    ``_lanes`` takes them for the block's length), or ``table``, used as it is, and the stream
+    count; returns how many blocks changed."""
+    lanes = _lanes if table is None else (lambda entry, team, quartets: entry)
     table = _load() if table is None else table
     configs = any(key.startswith(("v:", "c:")) for key in table)
     n = 0
-    for k, (cls4, team, avg, _) in enumerate(db.blocks()):
+    for k, (cls4, team, avg, quartets) in enumerate(db.blocks()):
         key = _key(cls4, avg)
         t = table.get(key)
-        if t and t != team:
+        t = lanes(t, team, quartets) if t else team
+        if t != team:
             db.set_team(k, int(t))
             n += 1
         if not configs:

@@ -76,13 +76,15 @@ class EriBatch:
     def apply_tuning(self, table=None):
         """Teams from the tuning cache (keyed by class and primitive bucket, shared with the
         single-basis tuner); returns how many types changed."""
-        from .autotune import _key, _load
+        from .autotune import _key, _lanes, _load
+        lanes = _lanes if table is None else (lambda entry, team, quartets: entry)
         table = _load() if table is None else table
         n = 0
-        for k, (cls4, team, avg, _) in enumerate(self.types()):
+        for k, (cls4, team, avg, quartets) in enumerate(self.types()):
             key = _key(cls4, avg)
             t = table.get(key)
-            if t and t != team:
+            t = lanes(t, team, quartets) if t else team
+            if t != team:
                 self.set_team(k, int(t))
                 n += 1
             v, c = table.get("v:" + key), table.get("c:" + key)

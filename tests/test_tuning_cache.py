@@ -78,6 +78,18 @@ def test_a_knob_moves_for_a_clear_gain_only(times, pick):
     assert autotune._pick((4, 8), times[1:], 2) == (4, 8)[times[2] < times[1]]
 
 
+@pytest.mark.parametrize("entry,team,quartets,lanes", [
+    (2, 16, 10, 16), (2, 16, 1200, 16), (2, 16, 2368, 16), (2, 16, 4736, 8), (2, 16, 9472, 4),
+    (2, 16, 18944, 2), (1, 4, 37887, 2), (1, 4, 37888, 1), (32, 16, 10, 32), (8, 8, 10, 8)])
+def test_short_lists_keep_the_lanes_that_fill_the_device(entry, team, quartets, lanes):
+    assert autotune._lanes(entry, team, quartets) == lanes
+
+
+def test_the_shipped_file_belongs_to_these_kernels(monkeypatch):
+    monkeypatch.delenv("GBX_TUNE_CACHE", raising=False)
+    assert autotune._load()
+
+
 def test_a_table_of_the_caller_is_used_as_it_is(cache):
     basis, batch = _Fake(), _Fake()
     autotune.apply_cache(basis, TABLE)
