@@ -598,12 +598,15 @@ def emit_sources(outdir, lmax):
         lines.append(f"int {rlaunchers[c]}(const EriLaunch& a, cudaStream_t st);")
     lines.append("// Heavy classes run the quadrature kernel (eri_rys) or, the smallest of them, the register kernel")
     lines.append("// (is_register in gen_eri.py); for both the block's variant knob selects the")
-    lines.append("// line kernel (1) or (2) its group form or, for the classes that have one, the split kernel:")
-    lines.append("// a thread per quartet, which is faster on long lists of quartets with equal primitive")
-    lines.append("// counts (33,000 to 120,000 quartets of 45 to 60 primitive quartets: 1.4 to 1.8 times,")
-    lines.append("// (pf|sp) 0.70 against 1.28 ms) and slower on short or uneven ones (7,000 to 20,000: 1.2")
-    lines.append("// to 1.9 times, (pd|sd) 0.31 against 0.19 ms).  The rule does not look at the list: a")
-    lines.append("// quartet's value must not depend on the list it is in.")
+    lines.append("// line kernel (1) or (2) its group form or, for the classes that have one, the split kernel.")
+    lines.append("// The split kernel, a thread per quartet, is faster on long lists of quartets with equal")
+    lines.append("// primitive counts and slower on short or uneven ones.  Its time over the quadrature kernel's")
+    lines.append("// on (pd|pp), (pd|sd), (pd|ds), (dp|pp), (dp|sd) and (dp|ds): 80,000 quartets 0.4 to 0.55 at")
+    lines.append("// one primitive quartet each and 0.6 to 0.7 at 81, 16,000 quartets 0.5 to 0.8 and 0.7 to 1.0,")
+    lines.append("// 700 quartets 1.7 and 1.7 to 2.6; of 1 to 256 primitive quartets, 16,000 quartets 1.3 to 1.8.")
+    lines.append("// It is the default on none: its recursion loses digits (error of these classes' values")
+    lines.append("// against 64-bit ones, split and quadrature: five atoms of s, p, d shells of one primitive")
+    lines.append("// 7.2e-16 and 2.5e-16, of four 1.8e-14 and 4.0e-15; a 5-atom batch molecule 2.6e-14 and 1.5e-14).")
     lines.append("// GBX_HEAVY_KERNEL=interp selects the")
     lines.append("// program-interpreting cooperative kernel instead (read once per process).")
     lines.append("static bool heavy_interp() {")

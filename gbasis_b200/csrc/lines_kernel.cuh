@@ -713,7 +713,7 @@ __device__ __forceinline__ void split_tail(const EriLaunch& a, double* ACC,
   }
 }
 
-// Split register kernel for heavy classes of moderate size: a CTA of S = C::kS warps (4 or 8)
+// Split register kernel for heavy classes of moderate size: a CTA of S = C::kS warps (4)
 // takes 32 quartets at a time, thread t of warp r computing part r (a contiguous range of bra
 // rows e) of quartet t's contracted [e0|f0] in registers (generated straight-line recursions,
 // as in the light classes' kernel); the parts meet in shared memory ACC[32][NE][RS] and all

@@ -15,13 +15,16 @@ import numpy as np
 import pytest
 
 from gbasis_b200 import _engine
-from gbasis_b200.autotune import light_class
 from gbasis_b200.batch import EriBatch
 from gbasis_b200.contractions import GeneralizedContractionShell
 
 pytestmark = pytest.mark.gpu
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+sys.path.insert(0, os.path.join(ROOT, "gbasis_b200", "csrc"))
+
+import gen_eri  # noqa: E402
+
 DEBUG_LIB = os.path.join(ROOT, "gbasis_b200", "_lib", "libgbx_eri_debug.so")
 
 
@@ -38,15 +41,12 @@ def _shells(coord, seed=11):
     return out
 
 
+# the classes that have variants: beyond one thread's registers in their own order
+HEAVY = {tuple(c) for c in gen_eri.canonical_classes(3) if not gen_eri.is_light(c)}
+
+
 def _heavy(blocks):
-    return [k for k, b in enumerate(blocks) if not light_class(b[0])]
-
-
-def _classes():
-    import sys as _sys
-    _sys.path.insert(0, os.path.join(ROOT, "gbasis_b200", "csrc"))
-    import gen_eri
-    return {tuple(c) for c in gen_eri.canonical_classes(3) if not gen_eri.is_register(c)}
+    return [k for k, b in enumerate(blocks) if b[0] in HEAVY]
 
 
 @pytest.mark.parametrize("coord", ["cartesian", "spherical"])
@@ -55,7 +55,7 @@ def test_variants_equal_the_default_kernels(variant, coord):
     import torch
     db = _engine.DeviceBasis(_shells(coord), tuned=False)
     heavy = _heavy(db.blocks())
-    assert {db.blocks()[k][0] for k in heavy} == _classes()
+    assert {db.blocks()[k][0] for k in heavy} == HEAVY
     n = db.nbf
     rng = np.random.default_rng(3)
     D = rng.uniform(-0.5, 0.5, (n, n))
