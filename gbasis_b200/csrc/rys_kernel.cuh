@@ -13,9 +13,9 @@
 // the sums go to shared memory ACC[e][f] once and the whole CTA runs the tail: horizontal
 // recursions, transforms, store / Schwarz maximum / Coulomb contributions.
 //
-// What bounds it: shared memory and the matrix pipe together (l1tex data pipe 64 to 69 %, FP64
-// matrix pipe 52 to 54 % on (dd|dd) and (df|sf) of 81 primitive quartets; (pd|sd) 69 and 34 %), with
-// the barriers between the phases.  The matrix instruction is there for its operand reuse:
+// What bounds it: shared memory and the matrix pipe together (l1tex data pipe 73 to 85 %, FP64
+// matrix pipe 53 to 58 % busy on 3,000 quartets of (dd|dd) and (df|fs) of 81 primitive quartets;
+// (ff|ff) 52 and 49 %), with the barriers between the phases.  The matrix instruction is there for its operand reuse:
 // the same sums with a lane per column and FMAs read 8 shared values for every 9 FMAs and took 1.4
 // to 2 times longer.  Measured on the 20-atom chain's first 10 atoms (spherical, unique integrals,
 // blocks one after another), the line or split kernel before against this one: all heavy classes
