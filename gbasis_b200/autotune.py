@@ -112,12 +112,20 @@ def _store(chosen):
 # this bound, twice it and four times it: one (dp|ps) quartet 0.60, 0.42, 0.42, 0.43 ms, resident s-f
 # chain of 7 atoms 6.75, 6.87, 6.96, 7.05 ms, 60-molecule batch 12.58, 12.57, 12.63, 12.68 ms.
 FILL = 148 * 256
+# Threads below which more lanes than the rule's pay: 148 SMs of 2 warps.  Where a list has more, the
+# call's other lists need the room (resident spd tensor of 8 atoms with entries above the rule on every
+# list, below FILL threads, below half, below a quarter, on none: 1.924, 1.909, 1.886, 1.871, 1.884 ms;
+# of 2 atoms 243, 239, 237, 238, 252 us).
+FEW = FILL // 4
 
 
 def _lanes(entry, team, quartets):
-    """Lanes per quartet for a block whose rule says ``team`` and whose cache entry is ``entry``: the
-    entry was measured on lists of 49,000 quartets and more, where fewer lanes leave less to add up;
-    a shorter list takes as many more, up to the rule's, as it needs to fill the device."""
+    """Lanes per quartet for a block whose rule says ``team`` and whose cache entry is ``entry``,
+    measured with the device to itself.  Fewer lanes than the rule's leave less to add up where the
+    list is long: a shorter one takes as many more, up to the rule's, as it needs to fill the
+    device.  More lanes shorten each quartet: only where the rule leaves the device nearly empty."""
+    if entry > team:
+        return entry if quartets * team < FEW else team
     while entry < team and quartets * entry < FILL:
         entry *= 2
     return entry

@@ -80,7 +80,8 @@ def test_a_knob_moves_for_a_clear_gain_only(times, pick):
 
 @pytest.mark.parametrize("entry,team,quartets,lanes", [
     (2, 16, 10, 16), (2, 16, 1200, 16), (2, 16, 2368, 16), (2, 16, 4736, 8), (2, 16, 9472, 4),
-    (2, 16, 18944, 2), (1, 4, 37887, 2), (1, 4, 37888, 1), (32, 16, 10, 32), (8, 8, 10, 8)])
+    (2, 16, 18944, 2), (1, 4, 37887, 2), (1, 4, 37888, 1), (32, 16, 10, 32), (32, 16, 591, 32),
+    (32, 16, 592, 16), (8, 8, 10, 8), (8, 8, 10 ** 6, 8)])
 def test_short_lists_keep_the_lanes_that_fill_the_device(entry, team, quartets, lanes):
     assert autotune._lanes(entry, team, quartets) == lanes
 
