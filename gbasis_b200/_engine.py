@@ -242,7 +242,8 @@ def pack_basis(shells, coord_types=None, raw=False):
             n_c, M, spherical = len(_SQRT_DFACT[l]), c.shape[1], ct == "spherical"
             nc = np.ones((M, n_c)) if raw else np.asarray(sh.norm_cont, dtype=float).reshape(M, n_c)
             n_o = 2 * l + 1 if spherical else n_c
-            if spherical and not (np.abs(nc - nc[:, :1]) <= 1e-14 * np.abs(nc[:, :1])).all():
+            if spherical and not (nc == nc[:, :1]).all() and not all(
+                    np.allclose(row, row[0], rtol=1e-14, atol=0) for row in nc):
                 raise NotImplementedError(
                     f"shell {si}: spherical transform with component-dependent norm_cont")
             center, e_list = np.asarray(sh.coord, dtype=float).ravel().tolist(), e.tolist()
